@@ -1,4 +1,6 @@
-// k_demag.cu — FFT demagnetising field for sm_100a, FP64.
+// k_demag.cu — FFT demagnetising field for sm_100a: the plan, the tensor
+// spectra, and the mixed-precision (FP32) chain; the FP64 chain is
+// k_demag64.cu, the mixed chain's tensor-core columns k_demag_tc.cu.
 //
 // Reference chain (src/irregular/2d_fft/2d_i2/demag_fft.cu:325-363, windowed
 // 2d_i3/demag_fft.cu:371-419):  gather (× w) → cufftExecD2Z (batch 3) →
@@ -6,7 +8,7 @@
 // scatter to SoA.  Tensor: 81-point face average of the closed-form Newell
 // integrals (demag_fft.cu:27-91) computed once at init.
 //
-// Here the chain is three hand-written kernels and no library FFT:
+// Here either chain is three hand-written kernels and no library FFT:
 //   K1 rows_fwd : SoA y (× w) → real FFT along x of each data row (two real
 //                 rows packed into one complex transform) → spectrum S written
 //                 column-major [comp][kx][y] so K2 reads whole columns.
@@ -15,14 +17,15 @@
 //                 inverse FFT along y → S (only the data rows are kept).
 //   K3 rows_inv : inverse real FFT along x → h, × strength/(Px·Py) folded into
 //                 the tensor, written SoA for the first ng columns only.
-// Every transform is a Stockham autosort FFT in shared memory (natural order
-// in and out, no reordering tables): each pass stages the thread's radix-R
-// butterflies in registers, synchronises, and scatters the results in place.
-// The lengths 1024/2048/3072/4096 run a compile-time plan (radix 16 first,
-// then one 12/8/6/4/2 pass; the kernels are instantiated per length, FIX),
-// every other length a runtime plan (radix 8/4/2/3/5, any other prime through
-// a generic path).  A CTA row of threads owns one transform; HBM sees each
-// element of y, S and h once per kernel.
+// The FP32 transforms here (and the FP64 ones that build the tensor spectra)
+// are Stockham autosort FFTs in shared memory (natural order in and out, no
+// reordering tables): each pass stages the thread's radix-R butterflies in
+// registers, synchronises, and scatters the results in place.  The lengths
+// 1024/2048/3072/4096 run a compile-time plan (radix 16 first, then one
+// 12/8/6/4/2 pass; the kernels are instantiated per length, FIX), every other
+// length a runtime plan (radix 8/4/2/3/5, any other prime through a generic
+// path).  A CTA row of threads owns one transform; HBM sees each element of
+// y, S and h once per kernel.
 // The tensor is stored wrapped at displacement d mod P (d in [-P/2, P-1-P/2]),
 // which equals the reference's centring + output shift; the open-boundary
 // tensor has its unused d = -P/2 lines zeroed, so its spectra are real.  Only
@@ -559,11 +562,7 @@ struct DemagPlan {
   double strength = 0.0;
   double n0[3] = {0, 0, 0};      // unscaled N(0)
   HostFft fx, fy;
-  double2* d_S = nullptr;        // 3*hx*ny
-  double* d_txx = nullptr;
-  double* d_tyy = nullptr;
-  double* d_tzz = nullptr;
-  double2* d_txy = nullptr;
+  double2* d_S = nullptr;        // 3*hx*ny (FP64 chain)
   double* d_T = nullptr;         // 9 real tensor components (kept for host queries)
   // mixed-precision chain (LLG_DEMAG_MIXED): FP32 spectrum and tensor spectra
   int mixed = 0;
@@ -572,7 +571,9 @@ struct DemagPlan {
   float* d_tyyf = nullptr;
   float* d_tzzf = nullptr;
   float2* d_txyf = nullptr;
-  LaunchCfg rows[2], cols[2];    // [0] FP64 chain, [1] FP32 chain (autotuned)
+  LaunchCfg rows, cols;          // launch shapes of the FP32 chain (autotuned)
+  int init_ept = 8;              // elements per thread of the FP64 row transform that builds the tensor spectra
+  Demag64* f64 = nullptr;        // FP64 chain (k_demag64.cu); null in the mixed form
   int* d_err = nullptr;          // wait-ran-out flag of the tensor-core column stage (the context's SLOT_TCERR)
   DemagTc* tc = nullptr;         // tensor-core column stage (k_demag_tc.cu), when the shape allows
   cudaGraphExec_t gexec = nullptr;   // captured chain for gkey = (y, w, h) on the context's own stream
@@ -645,10 +646,6 @@ void demag_destroy(DemagPlan* d) {
   fft_free(d->fx);
   fft_free(d->fy);
   cudaFree(d->d_S);
-  cudaFree(d->d_txx);
-  cudaFree(d->d_tyy);
-  cudaFree(d->d_tzz);
-  cudaFree(d->d_txy);
   cudaFree(d->d_T);
   cudaFree(d->d_Sf);
   cudaFree(d->d_txxf);
@@ -656,6 +653,7 @@ void demag_destroy(DemagPlan* d) {
   cudaFree(d->d_tzzf);
   cudaFree(d->d_txyf);
   demag_tc_destroy(d->tc);
+  demag64_destroy(d->f64);
   if (d->gexec) cudaGraphExecDestroy(d->gexec);
   delete d;
 }
@@ -668,9 +666,6 @@ static int set_smem(const void* fn, size_t bytes) {
 }
 
 // ── launch helpers (elements-per-thread dispatch) ─────────────────────────
-template <typename R>
-static constexpr int kp() { return sizeof(R) == 8 ? 0 : 1; }
-
 // Kernel of each launch shape: nb packed transforms per CTA, ept elements
 // per thread, and the compile-time plan of the transform length when it has
 // one (HostFft::fix).
@@ -781,6 +776,20 @@ static int launch_cols_conv(const DemagPlan* d, cudaStream_t s, cx_t<R>* S, cons
   return 0;
 }
 
+// one row pair per CTA, FP64, no padding (the tensor spectra at init)
+static RowsFwdFn<double> rows_fwd_init_fn(int fix, int ept) {
+  return ept == 8 ? rows_fwd_fn_t<double, 1, 8>(fix) : rows_fwd_fn_t<double, 1, 16>(fix);
+}
+static int launch_rows_fwd_init(const DemagPlan* d, cudaStream_t s, const double* in, int row_len, int nrows,
+                                double2* S) {
+  const FftPlan pl = d->fx.dev<double>();
+  const size_t sm = sizeof(double2) * (size_t)padded_len<double>(d->px);
+  klaunch(rows_fwd_init_fn(d->fx.fix, d->init_ept), dim3((nrows + 1) / 2, 1), dim3(d->fx.tx_for(d->init_ept), 1), sm, s,
+          pl, in, 0LL, row_len, nrows, (const double*)nullptr, S, d->py, d->hx);
+  LLG_CUDA_TRY(cudaPeekAtLastError());
+  return 0;
+}
+
 static int launch_cols_fwd(const DemagPlan* d, cudaStream_t s, double2* S) {
   const FftPlan pl = d->fy.dev<double>();
   const size_t sm = sizeof(double2) * (size_t)d->py;
@@ -796,6 +805,19 @@ static bool rows_ok(const DemagPlan* d, int nb, int ept) {
   return threads <= 1024 && sizeof(cx_t<R>) * (size_t)nb * padded_len<R>(d->px) <= 227 * 1024 &&
          threads <= max_threads((const void*)rows_fwd_fn<R>(d->fx.fix, nb, ept)) &&
          threads <= max_threads((const void*)rows_inv_fn<R>(d->fx.fix, nb, ept));
+}
+// Grids taken: the FP64 transforms' lengths, a limit of both chains (the
+// tensor spectra are built in FP64).  Rows up to one thread per 16 elements
+// and columns up to one per 16 of each component, within shared memory; a
+// prime factor above 5 counts one thread per butterfly.
+static int fits_f64(DemagPlan* d) {
+  const int r8 = d->fx.tx_for(8), r16 = d->fx.tx_for(16), c8 = d->fy.tx_for(8), c16 = d->fy.tx_for(16);
+  d->init_ept = (r8 <= 768 && r8 <= max_threads((const void*)rows_fwd_init_fn(d->fx.fix, 8))) ? 8 : 16;
+  const bool rows = (d->init_ept == 8 || r16 <= 512) && sizeof(double2) * (size_t)padded_len<double>(d->px) <= 227 * 1024;
+  const bool cols = (3 * c8 <= 896 || 3 * c16 <= 512 || c16 <= 256) && sizeof(double2) * 3 * (size_t)d->py <= 227 * 1024;
+  if (rows && cols) return 0;
+  llg_set_error("demag grid too large for the shared-memory transform");
+  return LLG_ERR_NOTSUP;
 }
 template <typename R>
 static size_t cols_smem(const DemagPlan* d, bool stage) {
@@ -832,8 +854,8 @@ static int set_smem_all(DemagPlan* d) {
   }
   // default shapes (before tuning): one transform per CTA, fewest elements
   // per thread that the kernel's registers allow
-  LaunchCfg& rw = d->rows[kp<R>()];
-  LaunchCfg& cl = d->cols[kp<R>()];
+  LaunchCfg& rw = d->rows;
+  LaunchCfg& cl = d->cols;
   rw.nb = 1;
   rw.ept = rows_ok<R>(d, 1, 8) ? 8 : 16;
   cl.cy = 3;
@@ -851,11 +873,11 @@ static int set_smem_all(DemagPlan* d) {
 // shapes as the three-kernel chain on this plan's buffers, keep the fastest.
 // All shapes compute bitwise-identical results (same butterflies, same
 // operation order per element), so tuning never changes numerics.  Results
-// are cached per (precision, transform size, grid) for later plans.
+// are cached per (transform size, grid) for later plans.
 struct TuneKey {
-  int prec, px, py, ny, ng;
+  int px, py, ny, ng;
   bool operator<(const TuneKey& o) const {
-    return std::tie(prec, px, py, ny, ng) < std::tie(o.prec, o.px, o.py, o.ny, o.ng);
+    return std::tie(px, py, ny, ng) < std::tie(o.px, o.py, o.ny, o.ng);
   }
 };
 static std::mutex g_tune_mu;
@@ -864,13 +886,13 @@ static std::map<TuneKey, std::pair<LaunchCfg, LaunchCfg>> g_tune;
 template <typename R>
 static int demag_autotune(llg_ctx* c, DemagPlan* d, cx_t<R>* S, const R* txx, const R* tyy, const R* tzz,
                           const cx_t<R>* txy, bool tune_cols) {
-  const TuneKey key{kp<R>(), d->px, d->py, d->ny, d->ng};
+  const TuneKey key{d->px, d->py, d->ny, d->ng};
   {
     std::lock_guard<std::mutex> g(g_tune_mu);
     auto it = g_tune.find(key);
     if (it != g_tune.end()) {
-      d->rows[kp<R>()] = it->second.first;
-      if (tune_cols) d->cols[kp<R>()] = it->second.second;
+      d->rows = it->second.first;
+      if (tune_cols) d->cols = it->second.second;
       return 0;
     }
   }
@@ -879,7 +901,7 @@ static int demag_autotune(llg_ctx* c, DemagPlan* d, cx_t<R>* S, const R* txx, co
   cudaEvent_t e0, e1;
   LLG_CUDA_TRY(cudaEventCreate(&e0));
   LLG_CUDA_TRY(cudaEventCreate(&e1));
-  LaunchCfg best_r = d->rows[kp<R>()], best_c = d->cols[kp<R>()];
+  LaunchCfg best_r = d->rows, best_c = d->cols;
   std::vector<LaunchCfg> rcand, ccand;
   for (int nb = 1; nb <= 2; nb++)
     for (int ept = 8; ept <= 16; ept *= 2) {
@@ -941,10 +963,10 @@ static int demag_autotune(llg_ctx* c, DemagPlan* d, cx_t<R>* S, const R* txx, co
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   LLG_CUDA_TRY(cudaGetLastError());
-  d->rows[kp<R>()] = best_r;
-  if (tune_cols) d->cols[kp<R>()] = best_c;
+  d->rows = best_r;
+  if (tune_cols) d->cols = best_c;
   std::lock_guard<std::mutex> g(g_tune_mu);
-  g_tune[key] = {best_r, tune_cols ? best_c : d->cols[kp<R>()]};
+  g_tune[key] = {best_r, tune_cols ? best_c : d->cols};
   return 0;
 }
 
@@ -982,7 +1004,9 @@ int demag_create(llg_ctx* c) {
     demag_destroy(d);
     return LLG_ERR_NOTSUP;
   }
-  if ((rc = set_smem_all<double>(d)) || (d->mixed && (rc = set_smem_all<float>(d))) ||
+  if ((rc = fits_f64(d)) || (d->mixed && (rc = set_smem_all<float>(d))) ||
+      (rc = set_smem((const void*)rows_fwd_init_fn(d->fx.fix, d->init_ept),
+                     sizeof(double2) * (size_t)padded_len<double>(d->px))) ||
       (rc = set_smem((const void*)cols_fwd_fn(d->fy.fix, 8), sizeof(double2) * (size_t)d->py)) ||
       (rc = set_smem((const void*)cols_fwd_fn(d->fy.fix, 16), sizeof(double2) * (size_t)d->py))) {
     demag_destroy(d);
@@ -990,11 +1014,6 @@ int demag_create(llg_ctx* c) {
   }
   const long long np = (long long)d->px * d->py;
   const long long nspec = (long long)d->hx * d->py;
-  LLG_CUDA_TRY(cudaMalloc(&d->d_S, sizeof(double2) * 3 * (size_t)d->hx * d->ny));
-  LLG_CUDA_TRY(cudaMalloc(&d->d_txx, sizeof(double) * nspec));
-  LLG_CUDA_TRY(cudaMalloc(&d->d_tyy, sizeof(double) * nspec));
-  LLG_CUDA_TRY(cudaMalloc(&d->d_tzz, sizeof(double) * nspec));
-  LLG_CUDA_TRY(cudaMalloc(&d->d_txy, sizeof(double2) * nspec));
   LLG_CUDA_TRY(cudaMalloc(&d->d_T, sizeof(double) * 9 * np));
 
   cudaStream_t s = c->stream;
@@ -1010,12 +1029,15 @@ int demag_create(llg_ctx* c) {
   d->n0[2] = n0[8];
 
   // spectra of all 9 components (real 2-D FFT: rows then columns)
+  // (the scaled FP64 spectra behind them: both chains keep copies in their own layout)
   double2* spec = nullptr;
-  LLG_CUDA_TRY(cudaMalloc(&spec, sizeof(double2) * 9 * (size_t)nspec));
+  LLG_CUDA_TRY(cudaMalloc(&spec, (sizeof(double2) * 10 + sizeof(double) * 3) * (size_t)nspec));
+  double2* const t_xy = spec + 9 * nspec;
+  double* const t_xx = reinterpret_cast<double*>(t_xy + nspec);
+  double* const t_yy = t_xx + nspec;
+  double* const t_zz = t_yy + nspec;
   for (int k = 0; k < 9; k++) {
-    LaunchCfg k1 = d->rows[kp<double>()];   // the default FP64 shape (one transform per CTA)
-    if ((rc = launch_rows_fwd<double>(d, s, d->d_T + k * np, 0, d->px, d->py, nullptr, spec + k * nspec, d->py, 1,
-                                      k1)) ||
+    if ((rc = launch_rows_fwd_init(d, s, d->d_T + k * np, d->px, d->py, spec + k * nspec)) ||
         (rc = launch_cols_fwd(d, s, spec + k * nspec))) {
       cudaFree(spec);
       demag_destroy(d);
@@ -1028,14 +1050,12 @@ int demag_create(llg_ctx* c) {
   const double scale = d->strength / (double)np;
   klaunch(k_tensor_finish, nblk, 256, 0, s, spec + 0 * nspec, spec + 4 * nspec, spec + 8 * nspec, spec + 1 * nspec,
                                        spec + 3 * nspec, spec + 2 * nspec, spec + 5 * nspec, spec + 6 * nspec,
-                                       spec + 7 * nspec, nspec, scale, d->d_txx, d->d_tyy, d->d_tzz, d->d_txy,
-                                       d_stats);
+                                       spec + 7 * nspec, nspec, scale, t_xx, t_yy, t_zz, t_xy, d_stats);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   std::vector<double> st(4 * nblk);
   LLG_CUDA_TRY(cudaMemcpyAsync(st.data(), d_stats, sizeof(double) * 4 * nblk, cudaMemcpyDeviceToHost, s));
   LLG_CUDA_TRY(cudaStreamSynchronize(s));
   cudaFree(d_stats);
-  cudaFree(spec);
   double mx[4] = {0, 0, 0, 0};
   for (int b = 0; b < nblk; b++)
     for (int k = 0; k < 4; k++) mx[k] = std::max(mx[k], st[4 * b + k]);
@@ -1046,6 +1066,7 @@ int demag_create(llg_ctx* c) {
              "demag tensor outside the film form: max|diag|=%.3e imag(diag)=%.3e |xz..|=%.3e |xy-yx|=%.3e", mx[0],
              mx[1], mx[2], mx[3]);
     llg_set_error(buf);
+    cudaFree(spec);
     c->demag = d;
     return LLG_ERR_NOTSUP;
   }
@@ -1055,45 +1076,34 @@ int demag_create(llg_ctx* c) {
     LLG_CUDA_TRY(cudaMalloc(&d->d_tyyf, sizeof(float) * nspec));
     LLG_CUDA_TRY(cudaMalloc(&d->d_tzzf, sizeof(float) * nspec));
     LLG_CUDA_TRY(cudaMalloc(&d->d_txyf, sizeof(float2) * nspec));
-    klaunch(k_tensor_to_f32, c->num_sms * 4, 256, 0, s, d->d_txx, d->d_tyy, d->d_tzz, d->d_txy, nspec, d->d_txxf,
-                                                   d->d_tyyf, d->d_tzzf, d->d_txyf);
+    klaunch(k_tensor_to_f32, c->num_sms * 4, 256, 0, s, t_xx, t_yy, t_zz, t_xy, nspec, d->d_txxf, d->d_tyyf,
+            d->d_tzzf, d->d_txyf);
     LLG_CUDA_TRY(cudaPeekAtLastError());
     // tensor-core column stage where the column shape allows it (else FP32 Stockham columns)
-    if ((rc = demag_tc_create(c, d->px, d->py, d->hx, d->ny, d->d_txxf, d->d_tyyf, d->d_tzzf, d->d_txyf, &d->tc))) {
-      c->demag = d;
-      return rc;
-    }
-    if ((rc = demag_autotune<float>(c, d, d->d_Sf, d->d_txxf, d->d_tyyf, d->d_tzzf, d->d_txyf, d->tc == nullptr))) {
-      c->demag = d;
-      return rc;
-    }
-  } else if ((rc = demag_autotune<double>(c, d, d->d_S, d->d_txx, d->d_tyy, d->d_tzz, d->d_txy, true))) {
-    c->demag = d;
-    return rc;
+    rc = demag_tc_create(c, d->px, d->py, d->hx, d->ny, d->d_txxf, d->d_tyyf, d->d_tzzf, d->d_txyf, &d->tc);
+    if (!rc)
+      rc = demag_autotune<float>(c, d, d->d_Sf, d->d_txxf, d->d_tyyf, d->d_tzzf, d->d_txyf, d->tc == nullptr);
+  } else {
+    LLG_CUDA_TRY(cudaMalloc(&d->d_S, sizeof(double2) * 3 * (size_t)d->hx * d->ny));
+    rc = demag64_create(c, d->px, d->py, d->hx, d->ng, d->ny, d->open, d->fx.d_tw, d->fy.d_tw, d->d_S, t_xx, t_yy,
+                        t_zz, t_xy, &d->f64);
   }
+  cudaFree(spec);   // (waits for the kernels that read it)
   c->demag = d;
-  return 0;
+  return rc;
 }
 
 // stage 0 rows_fwd, 1 column convolution, 2 rows_inv; FP64 or mixed chain
 static int demag_run_stage_raw(llg_ctx* c, DemagPlan* d, int stage, const double* y, const double* w, double* h) {
   const long long cs = (long long)c->ncell;
-  if (stage == 0) {
-    LLG_COUNT(KID_DEMAG_ROWS_FWD);
-    if (d->mixed) return launch_rows_fwd<float>(d, c->stream, y, cs, d->ng, d->ny, w, d->d_Sf, d->ny, 3, d->rows[1]);
-    return launch_rows_fwd<double>(d, c->stream, y, cs, d->ng, d->ny, w, d->d_S, d->ny, 3, d->rows[0]);
-  }
+  LLG_COUNT(stage == 0 ? KID_DEMAG_ROWS_FWD : stage == 1 ? KID_DEMAG_COLS : KID_DEMAG_ROWS_INV);
+  if (d->f64) return demag64_stage(c, d->f64, stage, y, w, h);
+  if (stage == 0) return launch_rows_fwd<float>(d, c->stream, y, cs, d->ng, d->ny, w, d->d_Sf, d->ny, 3, d->rows);
   if (stage == 1) {
-    LLG_COUNT(KID_DEMAG_COLS);
-    if (d->mixed) {
-      if (d->tc) return demag_tc_cols(c, d->tc, d->d_Sf);
-      return launch_cols_conv<float>(d, c->stream, d->d_Sf, d->d_txxf, d->d_tyyf, d->d_tzzf, d->d_txyf, d->cols[1]);
-    }
-    return launch_cols_conv<double>(d, c->stream, d->d_S, d->d_txx, d->d_tyy, d->d_tzz, d->d_txy, d->cols[0]);
+    if (d->tc) return demag_tc_cols(c, d->tc, d->d_Sf);
+    return launch_cols_conv<float>(d, c->stream, d->d_Sf, d->d_txxf, d->d_tyyf, d->d_tzzf, d->d_txyf, d->cols);
   }
-  LLG_COUNT(KID_DEMAG_ROWS_INV);
-  if (d->mixed) return launch_rows_inv<float>(d, c->stream, d->d_Sf, h, cs, d->rows[1]);
-  return launch_rows_inv<double>(d, c->stream, d->d_S, h, cs, d->rows[0]);
+  return launch_rows_inv<float>(d, c->stream, d->d_Sf, h, cs, d->rows);
 }
 
 // (timed when the family's live kernel timer is on)

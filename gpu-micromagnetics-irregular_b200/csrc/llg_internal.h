@@ -80,6 +80,7 @@ struct DevProblem {
 
 struct DemagPlan;   // k_demag.cu
 struct DemagTc;     // k_demag_tc.cu
+struct Demag64;     // k_demag64.cu
 struct Integrator;  // integrator.cu
 struct Learned;     // k_learned.cu
 
@@ -192,6 +193,15 @@ int demag_self(llg_ctx* c, double out3[3]);
 int demag_stage(llg_ctx* c, int stage, const double* y, double* h);
 int demag_dims(llg_ctx* c, int out[4]);
 int demag_tensor_host(llg_ctx* c, int comp, int dx, int dy, double* out);
+// FP64 chain on the in-place transforms (k_demag64.cu): stage 0 rows forward,
+// 1 columns, 2 rows inverse.  twx, twy: the lengths' twiddle tables (px, py
+// entries); S: the plan's spectrum buffer; txx..txy: FP64 tensor spectra, read
+// at creation only
+int demag64_create(llg_ctx* c, int px, int py, int hx, int ng, int ny, int open, const double2* twx, const double2* twy,
+                   double2* S, const double* txx, const double* tyy, const double* tzz, const double2* txy,
+                   Demag64** out);
+void demag64_destroy(Demag64* d);
+int demag64_stage(llg_ctx* c, Demag64* d, int stage, const double* y, const double* w, double* h);
 // tensor-core (tcgen05, FP16 hi+lo split, FP32 accumulation) column stage of the
 // mixed chain; *out stays null when the column shape is not supported
 int demag_tc_create(llg_ctx* c, int px, int py, int hx, int ny, const float* txx, const float* tyy,
