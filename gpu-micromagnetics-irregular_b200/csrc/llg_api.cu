@@ -242,6 +242,7 @@ int llg_set_mask(llg_ctx* c, const double* h_ymsk3) {
   }
   if (!c->d_act) LLG_CUDA_TRY(cudaMalloc(&c->d_act, n));
   LLG_CUDA_TRY(cudaMemcpy(c->d_act, act.data(), n, cudaMemcpyHostToDevice));
+  c->geom_version++;
   sync_dp(c);
   return 0;
 }
@@ -281,6 +282,7 @@ int llg_set_active_ids(llg_ctx* c, const int32_t* h_active, int32_t n_active, co
   c->n_inactive = n_inactive;
   if (!c->d_act) LLG_CUDA_TRY(cudaMalloc(&c->d_act, n));
   LLG_CUDA_TRY(cudaMemcpy(c->d_act, act.data(), n, cudaMemcpyHostToDevice));
+  c->geom_version++;
   sync_dp(c);
   return 0;
 }

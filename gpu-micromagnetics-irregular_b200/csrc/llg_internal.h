@@ -109,6 +109,7 @@ struct llg_ctx {
 
   // geometry
   uint8_t* d_act = nullptr;
+  int geom_version = 0;      // bumped whenever d_act is written
   int32_t* d_active_ids = nullptr;
   int32_t* d_inactive_ids = nullptr;
   int n_active = 0, n_inactive = 0;
@@ -219,7 +220,7 @@ int demag_check_last(llg_ctx* c);
 // ── learned preconditioner (k_learned.cu) ──────────────────────────────
 bool learned_active(llg_ctx* c);                 // LLG_PREC_LEARNED with weights, no fallback
 double* learned_zbuf(llg_ctx* c);                // 3N scratch for the block-Jacobi stage
-int learned_apply(llg_ctx* c, const double* ewt, double* out, int slot /* <0: no norm */);
+int learned_apply(llg_ctx* c, const double* ewt, double* out, int slot /* <0: no norm */, const double* z = nullptr);
 void learned_fall_back(llg_ctx* c, int reason /* 1 failed solve, 2 cost */);
 void learned_policy_record(llg_ctx* c, double it_learned, double it_bj, double kappa);
 bool learned_policy_on(llg_ctx* c);

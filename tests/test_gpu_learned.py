@@ -203,3 +203,42 @@ def test_fp32_basis_takes_over_when_the_network_is_dropped(gpu):
     assert l32["fell_back"] != 0 and l32["napply"] > 0
     assert not np.array_equal(y32, y64)
     assert np.isfinite(y32).all() and d64 <= 1e-3 and dref <= 1e-3
+
+
+@pytest.mark.parametrize("ng,ny", [(33, 17), (200, 150), (1000, 641)])
+def test_idle_tiles_of_the_fused_inference(gpu, ng, ny):
+    """Tiles without an active cell skip the network: the output stays that of
+    the layer-by-layer path (BF16 activations apart: 3 % of the largest
+    correction) on a mostly empty mask whose cells touch tile corners, exactly
+    zero on inactive cells, with the norm of what was written; also when the
+    output overwrites z, which the network reads around each cell."""
+    import torch
+    rng = np.random.default_rng(3)
+    mask = np.zeros((ny, ng))
+    for _ in range(6):
+        j, i = rng.integers(0, ny), rng.integers(0, ng)
+        mask[j:j + 5, i:i + 7] = 1.0
+    mask[0, 0] = mask[-1, -1] = mask[min(15, ny - 1), min(31, ng - 1)] = 1.0
+    theta = (rng.standard_normal(L.nparams()) * 0.15).astype(np.float32)
+    ctx = llg.Context(llg.default_params(ng, ny, precond_kind=llg.PREC_LEARNED))
+    ctx.set_mask(np.tile(mask.ravel(), 3))
+    ctx.learned_set_weights(theta)
+    n = ng * ny
+    z = torch.from_numpy(rng.standard_normal(3 * n)).cuda()
+    m = torch.from_numpy(rng.standard_normal(3 * n)).cuda()
+    ewt = torch.from_numpy(rng.uniform(0.5, 2.0, 3 * n)).cuda()
+    out = {}
+    for fused in (1, 0):
+        ctx.learned_set_fused(fused)
+        o = torch.full_like(z, float("nan"))
+        n2 = ctx.learned_apply(z, m, ewt, 0.03, o)
+        out[fused] = o
+        assert abs(n2 - float((o * o).sum())) <= 1e-10 * n2
+    on = torch.from_numpy(np.tile(mask.ravel(), 3)).cuda()
+    assert float((out[1] * (1 - on)).abs().max()) == 0.0
+    corr = float((out[0] - ewt * z * on).abs().max())
+    assert float((out[1] - out[0]).abs().max()) <= 3e-2 * corr
+    ctx.learned_set_fused(1)
+    zz = z.clone()
+    ctx.learned_apply(zz, m, ewt, 0.03, zz)
+    assert torch.equal(zz, out[1])
