@@ -23,6 +23,7 @@
 #include <math.h>
 #include <string.h>
 
+#include <utility>
 #include <vector>
 
 #include "llg_internal.h"
@@ -41,6 +42,7 @@ double powr(double b, double e) { return (b <= 0.0) ? 0.0 : pow(b, e); }
 
 struct Integrator {
   llg_ctx* c = nullptr;
+  cudaStream_t stream = nullptr;   // the context's stream of the last call
   long long neq = 0;
   int qmax = 5, maxl = 5, classical_gs = 1, mxstep = 500;
   // LLG_KRYLOV_FP32: the basis V[0..maxl] holds floats (the same allocations);
@@ -1225,24 +1227,47 @@ int integrator_create(llg_ctx* c, double t0, const double* y0, const llg_solver_
     return LLG_ERR_NOTSUP;
   }
   const size_t vb = sizeof(double) * (size_t)b->neq;
-  auto alloc = [&](double** p) -> int {
-    LLG_CUDA_TRY(cudaMalloc(p, vb));
-    LLG_CUDA_TRY(cudaMemsetAsync(*p, 0, vb, c->stream));
-    return 0;
-  };
-  int rc = 0;
-  for (int j = 0; j <= b->qmax && !rc; j++) rc = alloc(&b->zn[j]);
-  for (int j = 0; j <= b->maxl && !rc; j++) rc = alloc(&b->V[j]);
-  double** vs[] = {&b->ewt, &b->acor, &b->y, &b->tempv, &b->delta};
-  for (auto pp : vs)
-    if (!rc) rc = alloc(pp);
-  if (rc) { b->free_all(); delete b; return rc; }
-  if (y0 && cudaMemcpyAsync(b->zn[0], y0, vb, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess) {
+  // The vectors of the integrator that this one replaces are taken over where
+  // both have them (the context's grid, so their length, does not change): a
+  // film of 1536x512 holds 17 vectors of 18.9 MB, whose cudaMalloc and cudaFree
+  // cost 8 to 200 ms per call here against some 60 us for clearing them.  Until
+  // everything that can fail has succeeded, the old integrator is untouched.
+  Integrator* const old = c->integ;
+  std::vector<std::pair<double**, double**>> vs;   // (this one's, the old one's)
+  for (int j = 0; j <= b->qmax; j++) vs.push_back({&b->zn[j], old ? &old->zn[j] : nullptr});
+  for (int j = 0; j <= b->maxl; j++) vs.push_back({&b->V[j], old ? &old->V[j] : nullptr});
+  vs.push_back({&b->ewt, old ? &old->ewt : nullptr});
+  vs.push_back({&b->acor, old ? &old->acor : nullptr});
+  vs.push_back({&b->y, old ? &old->y : nullptr});
+  vs.push_back({&b->tempv, old ? &old->tempv : nullptr});
+  vs.push_back({&b->delta, old ? &old->delta : nullptr});
+  auto fail = [&](int rc) {
     b->free_all();
     delete b;
-    llg_set_error("integrator_init: copy of y0 failed");
-    return LLG_ERR_CUDA;
+    return rc;
+  };
+  for (auto& v : vs)
+    if (!(v.second && *v.second) && cudaMalloc(v.first, vb) != cudaSuccess) {
+      *v.first = nullptr;
+      llg_set_error("integrator_init: vector allocation failed");
+      cudaGetLastError();
+      return fail(LLG_ERR_CUDA);
+    }
+  // work of the old integrator on another stream may still use its vectors
+  if (old && old->stream != c->stream && cudaDeviceSynchronize() != cudaSuccess) {
+    llg_set_error("integrator_init: device synchronisation failed");
+    return fail(LLG_ERR_CUDA);
   }
+  double* const z0 = b->zn[0] ? b->zn[0] : old->zn[0];
+  if (y0 && cudaMemcpyAsync(z0, y0, vb, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess) {
+    llg_set_error("integrator_init: copy of y0 failed");
+    return fail(LLG_ERR_CUDA);
+  }
+  for (auto& v : vs) {
+    if (!*v.first) std::swap(*v.first, *v.second);
+    if (!(y0 && v.first == &b->zn[0])) LLG_CUDA_TRY(cudaMemsetAsync(*v.first, 0, vb, c->stream));
+  }
+  b->stream = c->stream;
   b->tn = t0;
   b->q = 1;
   b->L = 2;
@@ -1268,6 +1293,7 @@ void integrator_destroy(Integrator* b) {
 
 int integrator_run(llg_ctx* c, double tout, double* yout, double* tret) {
   if (!c->integ) { llg_set_error("llg_integrate before llg_integrator_init"); return LLG_ERR_STATE; }
+  c->integ->stream = c->stream;
   return c->integ->integrate(tout, yout, tret);
 }
 

@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <random>
+#include <type_traits>
 #include <vector>
 
 #include "dev_reduce.cuh"
@@ -809,36 +810,46 @@ int learned_harvest(llg_ctx* c, const double* u_src, const double* x, const doub
 }
 
 // ── training ──
+// one allocation (18 of them, and as many cudaFree, cost 2 to 8 ms a call)
 struct TrainBuf {
+  void* base = nullptr;
   float *u = nullptr, *m = nullptr, *ewt = nullptr, *x = nullptr, *mask = nullptr, *gam = nullptr;
   float *f = nullptr, *a1 = nullptr, *a2 = nullptr, *y3 = nullptr;
   float *d3 = nullptr, *d2 = nullptr, *d1 = nullptr, *part = nullptr;
+  float *w = nullptr, *g = nullptr;   // weights and gradient of llg_learned_loss_grad
   double *num = nullptr, *den = nullptr;
   PatchSrc* src = nullptr;
   int4* off = nullptr;
   void release() {
-    float* fs[] = {u, m, ewt, x, mask, gam, f, a1, a2, y3, d3, d2, d1, part};
-    for (float* p : fs) cudaFree(p);
-    cudaFree(num); cudaFree(den); cudaFree(src); cudaFree(off);
+    cudaFree(base);
+    cudaFree(src);
+    cudaFree(off);
   }
 };
 
 static int train_alloc(TrainBuf& t, int nb, int P) {
   const size_t pl = (size_t)nb * P * P;
   const int nblk = ((P + TW - 1) / TW) * ((P + TH - 1) / TH) * nb;
-  bool ok = cudaMalloc(&t.u, 4 * 3 * pl) == cudaSuccess && cudaMalloc(&t.m, 4 * 3 * pl) == cudaSuccess &&
-            cudaMalloc(&t.ewt, 4 * 3 * pl) == cudaSuccess && cudaMalloc(&t.x, 4 * 3 * pl) == cudaSuccess &&
-            cudaMalloc(&t.mask, 4 * pl) == cudaSuccess && cudaMalloc(&t.gam, 4 * nb) == cudaSuccess &&
-            cudaMalloc(&t.f, 4 * 9 * pl) == cudaSuccess && cudaMalloc(&t.a1, 4 * 16 * pl) == cudaSuccess &&
-            cudaMalloc(&t.a2, 4 * 16 * pl) == cudaSuccess && cudaMalloc(&t.y3, 4 * 3 * pl) == cudaSuccess &&
-            cudaMalloc(&t.d3, 4 * 3 * pl) == cudaSuccess && cudaMalloc(&t.d2, 4 * 16 * pl) == cudaSuccess &&
-            cudaMalloc(&t.d1, 4 * 16 * pl) == cudaSuccess &&
-            cudaMalloc(&t.part, 4 * (size_t)nblk * NW2) == cudaSuccess &&
-            cudaMalloc(&t.num, 8 * nb) == cudaSuccess && cudaMalloc(&t.den, 8 * nb) == cudaSuccess;
-  if (!ok) {
-    t.release();
-    llg_set_error("learned: training buffer allocation failed");
-    return LLG_ERR_NOMEM;
+  size_t off = 0;
+  auto take = [&](auto*& p, size_t n) {
+    p = reinterpret_cast<std::remove_reference_t<decltype(p)>>((char*)t.base + off);
+    off += (n * sizeof(*p) + 255) & ~(size_t)255;
+  };
+  for (int pass = 0; pass < 2; pass++) {   // sizes, then addresses
+    off = 0;
+    take(t.u, 3 * pl); take(t.m, 3 * pl); take(t.ewt, 3 * pl); take(t.x, 3 * pl);
+    take(t.mask, pl); take(t.gam, nb);
+    take(t.f, CIN0 * pl); take(t.a1, CH * pl); take(t.a2, CH * pl); take(t.y3, 3 * pl);
+    take(t.d3, 3 * pl); take(t.d2, CH * pl); take(t.d1, CH * pl);
+    take(t.part, (size_t)nblk * NW2);
+    take(t.w, NWT); take(t.g, NWT);
+    take(t.num, nb); take(t.den, nb);
+    if (pass == 0 && cudaMalloc(&t.base, off) != cudaSuccess) {
+      t.base = nullptr;
+      cudaGetLastError();
+      llg_set_error("learned: training buffer allocation failed");
+      return LLG_ERR_NOMEM;
+    }
   }
   return 0;
 }
@@ -1080,11 +1091,9 @@ int llg_learned_loss_grad(const float* h_w, int32_t nb, int32_t P, const float* 
   TrainBuf t;
   int rc = train_alloc(t, nb, P);
   if (rc) return rc;
-  float *w = nullptr, *g = nullptr;
+  float *const w = t.w, *const g = t.g;
   const size_t pl = (size_t)nb * P * P;
-  auto done = [&](int r) { t.release(); cudaFree(w); cudaFree(g); return r; };
-  if (cudaMalloc(&w, sizeof(float) * NWT) != cudaSuccess || cudaMalloc(&g, sizeof(float) * NWT) != cudaSuccess)
-    return done(LLG_ERR_NOMEM);
+  auto done = [&](int r) { t.release(); return r; };
   if (cudaMemcpy(w, h_w, sizeof(float) * NWT, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(t.u, h_u, 12 * pl, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(t.m, h_m, 12 * pl, cudaMemcpyHostToDevice) != cudaSuccess ||

@@ -292,3 +292,49 @@ def test_fp32_basis_with_an_inactive_learned_preconditioner_is_block_jacobi(gpu)
     assert np.array_equal(ya, yb)
     for k in COUNTERS:
         assert sa[k] == sb[k], k
+
+
+@pytest.mark.parametrize("first,second", [({}, {}), (dict(maxl=2, maxord=2), dict(maxl=7)), (dict(maxl=7), dict(maxl=2)),
+                                          (dict(krylov_precision=1, gs_type=1), {}), ({}, dict(krylov_precision=1, gs_type=1))])
+@pytest.mark.parametrize("streams", [False, True])
+def test_reinitialised_integrator_is_a_fresh_one(gpu, first, second, streams):
+    """A second integrator_init on a context takes over the first one's
+    vectors: the run that follows is bit for bit that of a fresh context,
+    whichever of the two is larger and whichever stream each ran on; an init
+    that is refused leaves the running integrator as it was."""
+    import torch
+    import llg
+    p = llg.default_params(70, 33, demag_mode=llg.DEMAG_OPEN, demag_strength=2.0, norm_kind=llg.NORM_REG)
+    rng = np.random.default_rng(1)
+    m = rng.standard_normal((3, 70 * 33))
+    y0 = torch.from_numpy((m / np.linalg.norm(m, axis=0)).ravel()).cuda()
+    torch.cuda.synchronize()
+
+    def run(ctx, opts, t):
+        out = torch.zeros_like(y0)
+        torch.cuda.synchronize()
+        ctx.integrator_init(0.0, y0, opts)
+        ctx.integrate(t, out)
+        return out
+
+    o1, o2 = llg.default_solver_opts(**first), llg.default_solver_opts(**second)
+    fresh = run(llg.Context(p), o2, 0.2)
+    torch.cuda.synchronize()
+    ctx = llg.Context(p)
+    s = torch.cuda.Stream()
+    run(ctx, o1, 0.3)
+    if streams:
+        llg.load().llg_set_stream(ctx.h, s.cuda_stream)
+    again = run(ctx, o2, 0.2)
+    torch.cuda.synchronize()
+    assert torch.equal(again, fresh)
+    bad = llg.default_solver_opts(gs_type=llg.GS_MODIFIED, krylov_precision=llg.KRYLOV_FP32)
+    with pytest.raises(llg.LLGError):
+        ctx.integrator_init(0.0, y0, bad)
+    a, b = torch.zeros_like(y0), torch.zeros_like(y0)
+    ctx.integrate(0.4, a)
+    other = llg.Context(p)
+    run(other, o2, 0.2)
+    other.integrate(0.4, b)
+    torch.cuda.synchronize()
+    assert torch.equal(a, b)
