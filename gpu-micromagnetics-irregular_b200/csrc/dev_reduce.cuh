@@ -18,8 +18,14 @@ constexpr int RT = 256;         // threads per reduction block
 constexpr int UB = 4;
 constexpr int RMAXB = 1024;     // max reduction blocks
 
+// One element per thread up to RMAXB blocks: a reduction over a small vector is
+// a chain of load, tree and last-block latencies, so more of them side by side
+// are free (24,576 unknowns: 96 blocks instead of the 12 of eight elements per
+// thread; 17 -> 6 us for V0 and its norm, 5.8 -> 4.7 ms for the 128x64 film's
+// first 2 time units, 28.3 -> 27.1 ms for a polycrystal of 720x400; two per
+// thread ran the same, four 5.1 and 27.9 ms).
 int red_blocks(long long n) {
-  long long b = (n + RT * 8 - 1) / (RT * 8);
+  long long b = (n + RT - 1) / RT;
   if (b > RMAXB) b = RMAXB;
   if (b < 1) b = 1;
   return (int)b;
