@@ -356,14 +356,7 @@ __global__ void __launch_bounds__(TX * TY, 4) k_arnoldi_tile(DevProblem P, const
 // field, the demag field of the centre cells.  The HBM reads of one tile
 // therefore overlap the FP64 work of the previous one instead of alternating
 // with it.  The gate of a cell is read ahead of the stencil wait, its stored
-// block inverse ahead of the stencil arithmetic.  One barrier per tile: a
-// thread scales the slots it copied itself, and the next copies start after
-// the barrier that also ends the previous tile (35.9 -> 34.8 us FP64 basis,
-// 29.7 -> 28.7 us FP32 basis at 1536x512, against three barriers and a
-// division per slot).  What bounds it is the latency of its 24 warps per SM
-// (issue 47 %, FP64 pipe 23 %, HBM 36 to 58 %): four CTAs spill (35.5 and
-// 34.9 us), and warps marching along y with their rows in registers need 128
-// of them (40.2 and 32.8 us).
+// block inverse ahead of the stencil arithmetic.
 constexpr int AP_SLOTS = (TY + 2) * TX + (TY + 2) * 2;   // staged stencil slots per component
 constexpr int AP_PLANE = (TY + 2) * (TX + 2);            // doubles per stencil component
 constexpr int AP_CELLS = TX * TY;
@@ -384,7 +377,7 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(sz) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
 __device__ __forceinline__ void ap_slot(int q, int& sx, int& sy) {
   if (q < (TY + 2) * TX) { sy = q / TX; sx = 1 + (q % TX); }
@@ -417,38 +410,27 @@ __global__ void __launch_bounds__(AP_NT, 3) k_arnoldi_pipe(DevProblem P, const V
   typedef double Plane[TY + 2][TX + 2];
   typedef float FPlane[TY + 2][TX + 2];
 
-  // this thread's slots (one, for some threads two), the same in every tile
-  constexpr int NS = (AP_SLOTS + AP_NT - 1) / AP_NT;
-  int sxs[NS], sys[NS];
-#pragma unroll
-  for (int i = 0; i < NS; i++) ap_slot(tid + i * AP_NT, sxs[i], sys[i]);
-  auto has = [&](int i) { return tid + i * AP_NT < AP_SLOTS; };
-  // start tile t's copies into B; bit i of the result: slot i lies on the grid
-  auto issue = [&](int t, double* B) -> unsigned {
+  auto issue = [&](int t, double* B) {
     const int x0 = (t % gx) * TX, y0 = (t / gx) * TY;
     Plane* Y = reinterpret_cast<Plane*>(B);
     Plane* V = Y + 3;
     Plane* S = Y + 6;
-    unsigned oks = 0u;
-#pragma unroll
-    for (int i = 0; i < NS; i++) {
-      if (!has(i)) break;
-      const int sx = sxs[i], sy = sys[i];
+    for (int q = tid; q < AP_SLOTS; q += AP_NT) {
+      int sx, sy;
+      ap_slot(q, sx, sy);
       int gi = x0 - 1 + sx, gj = y0 - 1 + sy;
       const bool ok = map_nb(gi, gj, ng, ny, P.bc);
-      const unsigned cell = ok ? (unsigned)(gj * ng + gi) : 0u;
-      oks |= (ok ? 1u : 0u) << i;
+      const long long cell = ok ? (long long)gj * ng + gi : 0;
 #pragma unroll
       for (int a = 0; a < 3; a++) {
-        const unsigned e = cell + (unsigned)(a * n);
-        cp_async8(&Y[a][sy][sx], y + e, ok);
+        cp_async8(&Y[a][sy][sx], y + a * (long long)n + cell, ok);
         if constexpr (F32) {
           FPlane* Fv = reinterpret_cast<FPlane*>(B + foff);
-          cp_async4(&Fv[a][sy][sx], in + e, ok);
+          cp_async4(&Fv[a][sy][sx], in + a * (long long)n + cell, ok);
         } else {
-          cp_async8(&V[a][sy][sx], in + e, ok);
+          cp_async8(&V[a][sy][sx], in + a * (long long)n + cell, ok);
         }
-        cp_async8(&S[a][sy][sx], s + e, ok);
+        cp_async8(&S[a][sy][sx], s + a * (long long)n + cell, ok);
       }
     }
     if (P.jv_full) {
@@ -459,46 +441,43 @@ __global__ void __launch_bounds__(AP_NT, 3) k_arnoldi_pipe(DevProblem P, const V
 #pragma unroll
       for (int a = 0; a < 3; a++) cp_async8(&C[a * AP_CELLS + tid], hd + a * (long long)n + cell, cok);
     }
-    return oks;
   };
 
   int t = blockIdx.x, b = 0;
-  unsigned oks = 0u;
-  if (t < ntiles) oks = issue(t, apsm);
+  if (t < ntiles) issue(t, apsm);
   cp_async_commit();
   for (; t < ntiles; t += gridDim.x, b ^= 1) {
     double* B = apsm + b * bufd;
+    const int tn = t + gridDim.x;
+    if (tn < ntiles) issue(tn, apsm + (b ^ 1) * bufd);
+    cp_async_commit();
     const int x0 = (t % gx) * TX, y0 = (t / gx) * TY;
     const int gi = x0 + tx, gj = y0 + ty;
     const bool cok = gi < ng && gj < ny;
     const int cell = gj * ng + gi;
     const double g = (cok && P.act) ? (P.act[cell] ? 1.0 : 0.0) : 1.0;   // gate, loaded while the tile lands
-    cp_async_wait0();
+    cp_async_wait1();
+    __syncthreads();
     Plane* Y = reinterpret_cast<Plane*>(B);
     Plane* V = Y + 3;
     Plane* S = Y + 6;
-    // vt = (ain in) / s on the slots that this thread copied itself (0 outside
-    // a free edge), so no barrier stands between the copies and this; the
-    // quotient as a product with the reciprocal
+    // vt = (ain in) / s on every staged slot (0 outside a free edge)
+    for (int q = tid; q < AP_SLOTS; q += AP_NT) {
+      int sx, sy;
+      ap_slot(q, sx, sy);
+      int ii = x0 - 1 + sx, jj = y0 - 1 + sy;
+      const bool ok = map_nb(ii, jj, ng, ny, P.bc);
+      if constexpr (F32) {
+        const FPlane* Fv = reinterpret_cast<const FPlane*>(B + foff);
 #pragma unroll
-    for (int i = 0; i < NS; i++) {
-      if (!has(i)) break;
-      const int sx = sxs[i], sy = sys[i];
-      const bool ok = (oks >> i) & 1u;
+        for (int a = 0; a < 3; a++)
+          V[a][sy][sx] = ok ? 1.0 * ((ain * (double)Fv[a][sy][sx]) / S[a][sy][sx]) : 0.0;
+      } else {
 #pragma unroll
-      for (int a = 0; a < 3; a++) {
-        double v;
-        if constexpr (F32) v = (double)reinterpret_cast<const FPlane*>(B + foff)[a][sy][sx];
-        else v = V[a][sy][sx];
-        V[a][sy][sx] = ok ? (ain * v) * __drcp_rn(S[a][sy][sx]) : 0.0;
+        for (int a = 0; a < 3; a++) V[a][sy][sx] = ok ? 1.0 * ((ain * V[a][sy][sx]) / S[a][sy][sx]) : 0.0;
       }
     }
-    // The tile's one barrier: its slots are ready, and every thread is done
-    // with the previous tile, so the other buffer can be refilled.
     __syncthreads();
-    const int tn = t + gridDim.x;
-    if (tn < ntiles) oks = issue(tn, apsm + (b ^ 1) * bufd);
-    cp_async_commit();
     if (cok) {
       double Pi[9];
       load_pinv(pinv, n, cell, Pi);   // first use after the stencil arithmetic below
@@ -547,6 +526,7 @@ __global__ void __launch_bounds__(AP_NT, 3) k_arnoldi_pipe(DevProblem P, const V
         out[2 * n + cell] = (VT)z2;
       }
     }
+    __syncthreads();   // buffer b is refilled by the next iteration's issue
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");   // (only empty groups remain)
 }
