@@ -18,20 +18,25 @@ constexpr int RT = 256;         // threads per reduction block
 constexpr int UB = 4;
 constexpr int RMAXB = 1024;     // max reduction blocks
 
-// One element per thread up to RMAXB blocks: a reduction over a small vector is
-// a chain of load, tree and last-block latencies, so more of them side by side
-// are free (24,576 unknowns: 96 blocks instead of the 12 of eight elements per
-// thread; 17 -> 6 us for V0 and its norm, 5.8 -> 4.7 ms for the 128x64 film's
-// first 2 time units, 28.3 -> 27.1 ms for a polycrystal of 720x400; two per
-// thread ran the same, four 5.1 and 27.9 ms).
-int red_blocks(long long n) {
-  long long b = (n + RT - 1) / RT;
+// Blocks of a reduction over n elements, per elements to a thread up to RMAXB
+// blocks.  per = 1 (llg_ctx::red_per) in the plain FP64 integrator: a reduction
+// over a small vector is a chain of load, tree and last-block latencies, so
+// more of them side by side are free (24,576 unknowns: 96 blocks instead of 12;
+// 17 -> 6 us for V0 and its norm, 5.8 -> 4.7 ms for the 128x64 film's first 2
+// time units, 28.3 -> 27.1 ms for a polycrystal of 720x400; two per thread ran
+// the same, four 5.1 and 27.9 ms).  per = 8 elsewhere: the entry points of
+// llg.h, whose sums callers may compare between contexts, and integrators with
+// FP32 parts, whose trajectories turn another rounding of a sum into other
+// FP32 values.
+constexpr int RED_PER = 8;
+int red_blocks(long long n, int per) {
+  long long b = (n + RT * per - 1) / (RT * per);
   if (b > RMAXB) b = RMAXB;
   if (b < 1) b = 1;
   return (int)b;
 }
 
-// red_blocks(n) capped at the blocks that are resident at once (per_sm of
+// red_blocks capped at the blocks that are resident at once (per_sm of
 // the kernel times the SMs): for kernels whose registers leave fewer than
 // red_blocks' count resident, each thread then takes more slice elements
 // instead of a second, partly filled wave running after the first.  The
@@ -50,8 +55,8 @@ inline int cap_resident(int b, int per_sm, int num_sms) {
   const long long cap = (long long)per_sm * num_sms;
   return (int)(b < cap ? b : cap);
 }
-inline int red_blocks_resident(long long n, int per_sm, int num_sms) {
-  return cap_resident(red_blocks(n), per_sm, num_sms);
+inline int red_blocks_resident(long long n, int per, int per_sm, int num_sms) {
+  return cap_resident(red_blocks(n, per), per_sm, num_sms);
 }
 // per_sm of one kernel, queried once per process (each expansion is its own
 // function-local static)

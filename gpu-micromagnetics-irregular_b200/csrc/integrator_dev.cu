@@ -1133,7 +1133,7 @@ struct Builder {
     const long long cap = (long long)c->num_sms * 8;
     return (int)(g > cap ? cap : (g < 1 ? 1 : g));
   }
-  int rb() const { return red_blocks(d->neq); }
+  int rb() const { return red_blocks(d->neq, c->red_per); }
   DState* S() const { return d->d_s; }
   const DevArgs* DA() const { return &d->d_s->da; }
   void launched(const char* what) { cu(cudaPeekAtLastError(), what); }

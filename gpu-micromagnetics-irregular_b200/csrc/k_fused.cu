@@ -45,8 +45,6 @@ struct ZPack {
   double* p[8];
 };
 
-int cell_blocks(int ncell) { return red_blocks(ncell); }
-
 __global__ void __launch_bounds__(RT) k_ewt_wrms(double rtol, double atol, const double* __restrict__ y,
                                                  double* __restrict__ ewt, long long n, double* partials,
                                                  unsigned int* counter, double* out, const DevArgs* da) {
@@ -557,7 +555,7 @@ int ew_blocks(const llg_ctx* c, long long n) {
 
 int fused_ewt_wrms(llg_ctx* c, double rtol, double atol, const double* y, double* ewt, int slot, const DevArgs* da) {
   LLG_COUNT(KID_REDUCE);
-  klaunch(k_ewt_wrms, red_blocks(c->neq), RT, 0, c->stream, rtol, atol, y, ewt, c->neq, c->d_red, c->d_counter,
+  klaunch(k_ewt_wrms, red_blocks(c->neq, c->red_per), RT, 0, c->stream, rtol, atol, y, ewt, c->neq, c->d_red, c->d_counter,
                                                        c->d_scal + slot, da);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   return 0;
@@ -606,7 +604,7 @@ static int psolve_scale_dot_impl(llg_ctx* c, const double* r, const double* ewt,
   LLG_COUNT(KID_PSOLVE);
   const float* pinvf = (sizeof(VT) == sizeof(float) && c->pinv_f32 && !da) ? reinterpret_cast<const float*>(c->d_pinv)
                                                                           : nullptr;
-  klaunch(k_psolve_scale_dot<VT>, cell_blocks(c->ncell), RT, 0, c->stream, c->dp, c->d_pm, c->d_ph, pinvf, r, ewt,
+  klaunch(k_psolve_scale_dot<VT>, red_blocks(c->ncell, c->red_per), RT, 0, c->stream, c->dp, c->d_pm, c->d_ph, pinvf, r, ewt,
           v0, c->gamma_setup, c->d_red, c->d_counter, c->d_scal + slot, da,
           slot_aout >= 0 ? c->d_scal + slot_aout : nullptr);
   LLG_CUDA_TRY(cudaPeekAtLastError());
@@ -629,7 +627,7 @@ static int lincomb_norm_impl(llg_ctx* c, int nv, const double* coef, const VT* c
   for (int k = 0; k < nv; k++) { cp.c[k] = coef[k]; xp.p[k] = X[k]; }
   const KScale kz{};
   LLG_COUNT(KID_REDUCE);
-  klaunch(k_lincomb_norm<VT>, red_blocks(c->neq), RT, 0, c->stream, nv, cp, xp, z, c->neq, c->d_red, c->d_counter,
+  klaunch(k_lincomb_norm<VT>, red_blocks(c->neq, c->red_per), RT, 0, c->stream, nv, cp, xp, z, c->neq, c->d_red, c->d_counter,
           c->d_scal + slot, ks ? *ks : kz);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   return 0;
@@ -670,7 +668,7 @@ int fused_update_wrms2(llg_ctx* c, bool ycor_zero, double* ycor, const double* d
   LLG_COUNT(KID_REDUCE);
   // (the device-resident form reads nothing back through the mailbox)
   const Pub pub = da ? Pub{} : take_publish(c);
-  klaunch(k_update_wrms2, red_blocks(c->neq), RT, 0, c->stream, ycor_zero ? nullptr : ycor, ycor, del, w, c->neq, c->d_red, c->d_counter,
+  klaunch(k_update_wrms2, red_blocks(c->neq, c->red_per), RT, 0, c->stream, ycor_zero ? nullptr : ycor, ycor, del, w, c->neq, c->d_red, c->d_counter,
                                                            c->d_scal + slot, da, pub);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   return 0;
@@ -679,7 +677,7 @@ int fused_update_wrms2(llg_ctx* c, bool ycor_zero, double* ycor, const double* d
 int fused_wrms2(llg_ctx* c, const double* x1, double a, const double* x2, double b, const double* x3,
                 const double* w, int slot) {
   LLG_COUNT(KID_REDUCE);
-  klaunch(k_wrms2, red_blocks(c->neq), RT, 0, c->stream, x1, a, x2, b, x3, w, c->neq, c->d_red, c->d_counter,
+  klaunch(k_wrms2, red_blocks(c->neq, c->red_per), RT, 0, c->stream, x1, a, x2, b, x3, w, c->neq, c->d_red, c->d_counter,
                                                     c->d_scal + slot);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   return 0;
@@ -695,12 +693,12 @@ static int lincomb_update_impl(llg_ctx* c, int nv, const double* coef, const VT*
   const KScale kz{};
   const KScale kk = ks ? *ks : kz;
   LLG_COUNT(KID_REDUCE);
-  const int nb = red_blocks(c->neq);
+  const int nb = red_blocks(c->neq, c->red_per);
   const double* yin = ycor_zero ? nullptr : ycor;
   double* out = c->d_scal + slot;
   const Pub pub = take_publish(c);
 #define LU_K(NV)                                                                                                   \
-  klaunch(k_lincomb_update_k<NV, VT>, red_blocks_resident(c->neq, LLG_PER_SM((k_lincomb_update_k<NV, VT>)), c->num_sms), \
+  klaunch(k_lincomb_update_k<NV, VT>, red_blocks_resident(c->neq, c->red_per, LLG_PER_SM((k_lincomb_update_k<NV, VT>)), c->num_sms), \
           RT, 0, c->stream, cp, xp, w, del, yin, ycor, c->neq, c->d_red, c->d_counter, out, kk, pub)
   switch (nv) {
     case 1: LU_K(1); break;
@@ -771,7 +769,7 @@ int fused_complete(llg_ctx* c, int q, int qmax, const double* l, const double* a
   LLG_COUNT(KID_ELEMWISE);
   const int sv = save ? 1 : 0, nm = norms ? 1 : 0, st = store ? 1 : 0;
 #define COMP(Q)                                                                                    \
-  klaunch(k_complete_norms<Q>, red_blocks_resident(c->neq, LLG_PER_SM((k_complete_norms<Q>)), c->num_sms), RT, 0, \
+  klaunch(k_complete_norms<Q>, red_blocks_resident(c->neq, c->red_per, LLG_PER_SM((k_complete_norms<Q>)), c->num_sms), RT, 0, \
           c->stream, qmax, lp, acor, zp, zn[qmax], sv, nm, -cquot,                                                   \
                                                                 w, c->neq, c->d_red, c->d_counter,             \
                                                                 c->d_scal + slot, st)

@@ -750,7 +750,7 @@ int learned_apply(llg_ctx* c, const double* ewt, double* out, int slot, const do
   k_feat_grid<<<c->num_sms * 8, 256, 0, c->stream>>>(z, c->d_pm, c->d_act, n, l->d_f);
   if ((rc = net_forward(c->stream, l->d_wq, l->d_f, l->d_a1, l->d_a2, l->d_y3, 1, c->p.ny, c->p.ng))) return rc;
   LLG_COUNT(KID_LEARNED);
-  k_combine<<<red_blocks(n), RT, 0, c->stream>>>(z, l->d_y3, ewt, c->d_act, c->gamma_setup, n, out, c->d_red,
+  k_combine<<<red_blocks(n, RED_PER), RT, 0, c->stream>>>(z, l->d_y3, ewt, c->d_act, c->gamma_setup, n, out, c->d_red,
                                                 c->d_counter, slot >= 0 ? c->d_scal + slot : nullptr);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   l->napply++;

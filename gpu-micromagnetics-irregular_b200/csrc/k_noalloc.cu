@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(NA_T) k_dot_multi_noalloc(const double* __rest
 }
 
 int na_blocks(long long n) {
-  long long b = (n + NA_T - 1) / NA_T;
+  long long b = (n + NA_T * 8 - 1) / (NA_T * 8);
   if (b > NA_MAXB) b = NA_MAXB;
   if (b < 1) b = 1;
   return (int)b;

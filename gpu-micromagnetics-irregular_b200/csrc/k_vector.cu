@@ -394,7 +394,7 @@ static int vdot_multi_impl(llg_ctx* c, int nvec, const VT* x, const VT* const* Y
   VPack<VT> pk{};
   for (int k = 0; k < nvec; k++) pk.p[k] = Y[k];
   const long long n = c->neq;
-  const int nb = red_blocks(n);
+  const int nb = red_blocks(n, c->red_per);
   double* out = c->d_scal + slot;
   switch (nvec) {
 #define DOTK(K) \
@@ -417,7 +417,7 @@ int vdot_multi_dev_f(llg_ctx* c, int nvec, const float* x, const float* const* Y
 int vwrms_dev(llg_ctx* c, const double* x, const double* w, int slot) {
   const long long n = c->neq;
   LLG_COUNT(KID_REDUCE);
-  klaunch(k_wrms, red_blocks(n), RT, 0, c->stream, x, w, n, c->d_red, c->d_counter, c->d_scal + slot);
+  klaunch(k_wrms, red_blocks(n, c->red_per), RT, 0, c->stream, x, w, n, c->d_red, c->d_counter, c->d_scal + slot);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   return 0;
 }
@@ -425,7 +425,7 @@ int vwrms_dev(llg_ctx* c, const double* x, const double* w, int slot) {
 int vwrms_diff_dev(llg_ctx* c, double a, const double* x, double b, const double* y, const double* w, int slot) {
   const long long n = c->neq;
   LLG_COUNT(KID_REDUCE);
-  klaunch(k_wrms_lin, red_blocks(n), RT, 0, c->stream, a, x, b, y, w, n, c->d_red, c->d_counter, c->d_scal + slot);
+  klaunch(k_wrms_lin, red_blocks(n, c->red_per), RT, 0, c->stream, a, x, b, y, w, n, c->d_red, c->d_counter, c->d_scal + slot);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   return 0;
 }
@@ -492,14 +492,14 @@ static int vgs_update_impl(llg_ctx* c, int k, VT* const* V, int slot_dots, int s
   for (int j = 0; j < k; j++) pk.p[j] = V[j];
   const KScale kz{};
   LLG_COUNT(KID_REDUCE);
-  const int nb = red_blocks(c->neq);
+  const int nb = red_blocks(c->neq, c->red_per);
   const double* dots = c->d_scal + slot_dots;
   double* ss = c->d_scal + slot_ss;
   double* aout = slot_aout >= 0 ? c->d_scal + slot_aout : nullptr;
   const KScale kk = ks ? *ks : kz;
   const Pub pub = take_publish(c);
 #define GS_K(K)                                                                                                  \
-  klaunch(k_gs_update_k<K, VT>, red_blocks_resident(c->neq, LLG_PER_SM((k_gs_update_k<K, VT>)), c->num_sms), RT, \
+  klaunch(k_gs_update_k<K, VT>, red_blocks_resident(c->neq, c->red_per, LLG_PER_SM((k_gs_update_k<K, VT>)), c->num_sms), RT, \
           0, c->stream, pk, dots, V[k], c->neq, c->d_red, c->d_counter, ss, kk, aout, pub)
   switch (k) {
     case 1: GS_K(1); break;
@@ -632,7 +632,7 @@ int vscale_columns_f(llg_ctx* c, int q, const double* f, double* const* zn) {
 int vset_ewt(llg_ctx* c, double rtol, double atol, const double* y, double* ewt, int slot) {
   const long long n = c->neq;
   LLG_COUNT(KID_REDUCE);
-  klaunch(k_set_ewt, red_blocks(n), RT, 0, c->stream, rtol, atol, y, ewt, n, c->d_red, c->d_counter, c->d_scal + slot);
+  klaunch(k_set_ewt, red_blocks(n, c->red_per), RT, 0, c->stream, rtol, atol, y, ewt, n, c->d_red, c->d_counter, c->d_scal + slot);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   return 0;
 }
@@ -640,7 +640,7 @@ int vhin_bound(llg_ctx* c, double rtol, double atol, const double* y0, const dou
   (void)tmp;
   const long long n = c->neq;
   LLG_COUNT(KID_REDUCE);
-  klaunch(k_hin_bound, red_blocks(n), RT, 0, c->stream, rtol, atol, y0, f0, n, c->d_red, c->d_counter, c->d_scal + 40);
+  klaunch(k_hin_bound, red_blocks(n, c->red_per), RT, 0, c->stream, rtol, atol, y0, f0, n, c->d_red, c->d_counter, c->d_scal + 40);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   return 0;
 }

@@ -92,6 +92,15 @@ static int validate(const llg_params* p) {
   return 0;
 }
 
+// the reductions of llg.h sum on one partition whatever integrator the
+// context holds
+struct PublicReduction {
+  llg_ctx* c;
+  int saved;
+  explicit PublicReduction(llg_ctx* ctx) : c(ctx), saved(ctx->red_per) { c->red_per = 8; }
+  ~PublicReduction() { c->red_per = saved; }
+};
+
 void ktimer_mark(llg_ctx* c, int kid, bool pre) {
   if (!(c->timer_mask & (1u << kid)) || !c->timer_ev || c->capturing) return;
   int& k = c->timer_n[kid];
@@ -378,6 +387,7 @@ const double* llg_hdemag_device(llg_ctx* c) { return c ? c->d_hd : nullptr; }
 
 int llg_dot_multi(llg_ctx* c, int nvec, const double* d_x, const double* const* d_Y, double* h_out) {
   if (!c || !d_x || !d_Y || !h_out || nvec < 1 || nvec > 16) return LLG_ERR_ARG;
+  const PublicReduction pr(c);
   int rc = vdot_multi_dev(c, nvec, d_x, d_Y, 8);
   if (rc) return rc;
   return fetch_scalars(c, 8, nvec, h_out);
@@ -390,6 +400,7 @@ int llg_linear_combination(llg_ctx* c, int nvec, const double* coef, const doubl
 
 int llg_wrms_norm(llg_ctx* c, const double* d_x, const double* d_w, double* h_out) {
   if (!c || !d_x || !d_w || !h_out) return LLG_ERR_ARG;
+  const PublicReduction pr(c);
   int rc = vwrms_dev(c, d_x, d_w, 0);
   if (rc) return rc;
   return fetch_scalars(c, 0, 1, h_out);

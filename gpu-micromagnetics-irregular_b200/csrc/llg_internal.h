@@ -141,6 +141,7 @@ struct llg_ctx {
   Pub pub_armed{};              // requested, not yet given to a launch
   Pub pub_carried{};            // given to the last launch that took one
   int red_blocks_max = 0;
+  int red_per = 8;              // elements per thread of a reduction (red_blocks); set by integrator_create
 
   DemagPlan* demag = nullptr;
   Integrator* integ = nullptr;
