@@ -294,7 +294,7 @@ struct Integrator {
   bool fuse_update = false, update_done = false;   // see nls_lsolve / newton
   double upd_s[2] = {0.0, 0.0};
 
-  // ── read-back-light SPGMR (classical Gram-Schmidt, block-Jacobi) ──
+  // ── read-back-light SPGMR (block-Jacobi; either Gram-Schmidt) ──
   // The Arnoldi iterations of one solve are enqueued with every coefficient
   // formed on the device (V0 / ||V0||, the Gram-Schmidt update from its own
   // dots, V[k] / ||V[k]||), and the first two are enqueued before any read-
@@ -334,6 +334,19 @@ struct Integrator {
       ok(vgs_update_dev_f(c, k, W, slot_it(l), slot_ss(l), &ys, slot_sc(l)));
     } else {
       ok(launch_arnoldi_op(c, V[l], ewt, V[k], y, gamma, 1, nullptr, ka[l]));
+      if (!classical_gs) {   // ||V[k]||^2, then every coefficient from the updated V[k]
+        const double* Y2[2] = {V[k], V[0]};
+        const KScale y2{{nullptr, ka[0]}};
+        ok(vdot_multi_dev(c, 2, V[k], Y2, slot_it(l), &y2));
+        for (int i = 0; i < k; i++) {
+          const bool last = i + 1 == k;
+          if (last && pub_lo >= 0) arm_publish(c, pub_lo, slot_ss(l) + 1);
+          ok(vmgs_step_dev(c, V[i], ka[i], slot_it(l) + 1 + i, last ? nullptr : V[i + 1], last ? nullptr : ka[i + 1],
+                           V[k], last ? slot_ss(l) : slot_it(l) + 2 + i, slot_it(l), last ? slot_sc(l) : -1));
+        }
+        ka[k] = c->d_scal + slot_sc(l);
+        return;
+      }
       const double* Y[MAXLL + 1];
       for (int i = 0; i <= k; i++) Y[i] = V[i];
       ok(vdot_multi_dev(c, k + 1, V[k], Y, slot_it(l), &ys));
@@ -379,12 +392,38 @@ struct Integrator {
       njv++;
       nps++;
       const int k = l + 1;
-      const double* d = hsc + slot_it(l);
-      const double vk_norm = sqrt(d[k]);
+      // classical: the k coefficients, then ||V[k]||^2; modified: ||V[k]||^2 first
+      const double* d = hsc + slot_it(l) + (classical_gs ? 0 : 1);
+      const double vk_norm = sqrt(classical_gs ? d[k] : d[-1]);
       for (int i = 0; i < k; i++) Hes[i][l] = d[i];
       double nrm = sqrt(hsc[slot_ss(l)]);
       bool second = false;
-      if (GS_FACTOR * nrm < vk_norm) {
+      if (!classical_gs) {
+        double temp = GS_FACTOR * vk_norm;
+        if ((temp + nrm) == temp) {   // (V[k]'s scale is 1: the device made the same test)
+          second = true;
+          queued = k;
+          double nn2 = 0.0;
+          for (int i = 0; i < k; i++) {
+            const double* Y1[1] = {V[i]};
+            const KScale y1{{ka[i]}};
+            double np = 0.0, ss = 0.0;
+            if (ok(vdot_multi_dev(c, 1, V[k], Y1, SLOT_DOTS, &y1))) ok(fetch_scalars(c, SLOT_DOTS, 1, &np));
+            temp = GS_FACTOR * Hes[i][l];
+            if ((temp + np) == temp) continue;
+            Hes[i][l] += np;
+            const double cf[2] = {1.0, -np};
+            const double* X[2] = {V[k], V[i]};
+            const KScale x1{{nullptr, ka[i]}};
+            if (ok(fused_lincomb_norm(c, 2, cf, X, V[k], SLOT_DOTS, &x1))) ok(fetch_scalars(c, SLOT_DOTS, 1, &ss));
+            nn2 += np * np;
+          }
+          if (nn2 != 0.0) {
+            const double t2 = nrm * nrm - nn2;
+            nrm = (t2 > 0.0) ? sqrt(t2) : 0.0;
+          }
+        }
+      } else if (GS_FACTOR * nrm < vk_norm) {
         // second pass; V[k]'s scale is 1 (the device made the same test),
         // so later queued iterations are void and are enqueued again
         second = true;
@@ -454,7 +493,7 @@ struct Integrator {
     const bool harvest = !learned && learned_harvest_wanted(c);
     double* zb = (learned || harvest) ? learned_zbuf(c) : nullptr;
     if ((learned || harvest) && !zb) return LS_CONV_FAIL;
-    if (!learned && classical_gs) return spgmr_spec(rhs, delta_tol, harvest, zb);
+    if (!learned) return spgmr_spec(rhs, delta_tol, harvest, zb);
     if (kf32) { llg_set_error("FP32 Krylov basis: the learned / modified Gram-Schmidt solver keeps FP64"); err = LLG_ERR_NOTSUP; return LS_CONV_FAIL; }
     nps++;
     double ss = 0.0;

@@ -333,6 +333,45 @@ __global__ void __launch_bounds__(RT) k_gs_update_k(VPack<VT> X, const double* _
   if (last) publish_carried(pub);
 }
 
+// One step of modified Gram-Schmidt with its coefficient read on the device:
+// z = 1 z + (-*hd) (xa X), and the next coefficient's sum z (ya Y) or, after the
+// last step (Y null), z z.  Per element and per product the operations of the
+// separate pass and dot product, without the read-back between them.
+__global__ void __launch_bounds__(RT) k_mgs_step(const double* __restrict__ X, const double* xa_p,
+                                                 const double* __restrict__ hd, const double* __restrict__ Y,
+                                                 const double* ya_p, double* z, long long n, double* partials,
+                                                 unsigned int* counter, double* out, const double* vk, double* aout,
+                                                 Pub pub) {
+  pdl_entry();
+  __shared__ double sm[RT / 32];
+  const double h = *hd, xa = kscale_of(xa_p), ya = kscale_of(ya_p);
+  double acc[1] = {0.0};
+  const long long st = (long long)gridDim.x * RT;
+  for (long long i0 = blockIdx.x * (long long)RT + threadIdx.x; i0 < n; i0 += UB * st) {
+    double zv[UB], xv[UB], yv[UB];
+#pragma unroll
+    for (int u = 0; u < UB; u++) {
+      const long long i = i0 + u * st;
+      const bool in = i < n;
+      zv[u] = in ? z[i] : 0.0;
+      xv[u] = in ? X[i] : 0.0;
+      yv[u] = (in && Y) ? Y[i] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < UB; u++) {
+      const long long i = i0 + u * st;
+      if (i >= n) continue;
+      const double s = (-h) * (xa * xv[u]) + 1.0 * zv[u];
+      z[i] = s;
+      acc[0] += s * (Y ? ya * yv[u] : s);
+    }
+  }
+  block_sum<1>(acc, sm);
+  const bool last = finalize<1>(partials, gridDim.x, counter, out, 0, 1.0, acc);
+  if (last && aout && threadIdx.x == 0) *aout = mgs_scale_of(out[0], *vk);
+  if (last) publish_carried(pub);
+}
+
 // one warp copies d_scal[lo, hi) into the mapped host mailbox, makes the
 // copies visible to the host, then writes the sequence word last
 __global__ void k_publish(const double* __restrict__ src, int lo, int hi, double* mail,
@@ -525,6 +564,18 @@ int vgs_update_dev(llg_ctx* c, int k, double* const* V, int slot_dots, int slot_
 int vgs_update_dev_f(llg_ctx* c, int k, float* const* V, int slot_dots, int slot_ss, const KScale* ks,
                      int slot_aout) {
   return vgs_update_impl<float>(c, k, V, slot_dots, slot_ss, ks, slot_aout);
+}
+
+int vmgs_step_dev(llg_ctx* c, const double* X, const double* xa, int slot_h, const double* Y, const double* ya, double* z,
+                  int slot_out, int slot_vk, int slot_aout) {
+  LLG_COUNT(KID_REDUCE);
+  const Pub pub = take_publish(c);
+  klaunch(k_mgs_step, red_blocks(c->neq, c->red_per), RT, 0, c->stream, X, xa,
+          (const double*)(c->d_scal + slot_h), Y, ya, z, c->neq, c->d_red, c->d_counter, c->d_scal + slot_out,
+          (const double*)(slot_aout >= 0 ? c->d_scal + slot_vk : nullptr),
+          slot_aout >= 0 ? c->d_scal + slot_aout : (double*)nullptr, pub);
+  LLG_CUDA_TRY(cudaPeekAtLastError());
+  return 0;
 }
 
 int fetch_scalars(llg_ctx* c, int slot, int n, double* out) {

@@ -251,6 +251,12 @@ __device__ __forceinline__ double gs_scale_of(double ss, const double* vk) {
   if (vk && 1000.0 * sqrt(ss) < sqrt(*vk)) return 1.0;
   return 1.0 / sqrt(ss);
 }
+// the same after modified Gram-Schmidt, whose second pass is due when ||v||
+// vanishes against 1000 ||v before|| (rounded as the host's test)
+__device__ __forceinline__ double mgs_scale_of(double ss, double vk) {
+  const double nrm = sqrt(ss), temp = __dmul_rn(1000.0, sqrt(vk));
+  return __dadd_rn(temp, nrm) != temp ? 1.0 / nrm : 1.0;
+}
 #endif
 
 // device-side: results land in c->d_scal[slot..]; host copy via fetch_scalars
@@ -274,6 +280,11 @@ Pub take_publish(llg_ctx* c);
 // the vector's pre-update sum of squares at d_scal[slot_dots + k])
 int vgs_update_dev(llg_ctx* c, int k, double* const* V, int slot_dots, int slot_ss, const KScale* ks = nullptr,
                    int slot_aout = -1);
+// modified Gram-Schmidt: z -= d_scal[slot_h] (xa X), then d_scal[slot_out] = z .
+// (ya Y), or z . z (Y null) with z's KScale scale to slot_aout, judged against
+// its sum of squares before the first step at slot_vk
+int vmgs_step_dev(llg_ctx* c, const double* X, const double* xa, int slot_h, const double* Y, const double* ya, double* z,
+                  int slot_out, int slot_vk = 0, int slot_aout = -1);
 // FP32 Krylov basis (LLG_KRYLOV_FP32): the basis is stored as float, every
 // product and sum is formed in FP64
 int vdot_multi_dev_f(llg_ctx* c, int nvec, const float* x, const float* const* Y, int slot,

@@ -338,3 +338,36 @@ def test_reinitialised_integrator_is_a_fresh_one(gpu, first, second, streams):
     other.integrate(0.4, b)
     torch.cuda.synchronize()
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("ng,ny,win", [(5, 3, 0), (96, 48, 0), (130, 65, 1)])
+@pytest.mark.parametrize("maxl", [1, 3, 5])
+def test_modified_gram_schmidt_takes_the_oracles_steps(gpu, oracle_lib, ng, ny, win, maxl):
+    """Modified Gram-Schmidt with its coefficients formed on the device, against
+    the oracle's (one dot product and one pass at a time): the same step,
+    Newton and Krylov counts and the state within the parity tests' 1e-6."""
+    import torch
+    p = llg.default_params(ng, ny, demag_mode=llg.DEMAG_OPEN, demag_strength=3.0, norm_kind=llg.NORM_REG, windowed=win)
+    rng = np.random.default_rng(ng)
+    m = rng.standard_normal((3, ng * ny)) * 0.3
+    m[0] += 1.0
+    y0 = (m / np.linalg.norm(m, axis=0)).ravel()
+    ctx, o = llg.Context(p), oracle_lib.Oracle(p)
+    if win:
+        w = rng.uniform(0.2, 1.0, ng * ny)
+        axes = np.tile([1.0, 0.0, 0.0], (ng * ny, 1)).T.ravel().copy()
+        ctx.set_window(w, axes, axes)
+        o.set_window(w, axes, axes)
+    opts = llg.default_solver_opts(gs_type=llg.GS_MODIFIED, maxl=maxl)
+    ctx.integrator_init(0.0, torch.from_numpy(y0).cuda(), opts)
+    o.integrator_init(y0.copy(), opts)
+    out = torch.zeros(3 * ng * ny, dtype=torch.float64, device="cuda")
+    for k in (1, 2, 3):
+        ctx.integrate(0.1 * k, out)
+        rc, _, yo = o.integrate(0.1 * k)
+        assert rc == 0
+    torch.cuda.synchronize()
+    st, so = ctx.stats(), o.stats()
+    for k in ("nst", "nfe", "nni", "nli", "netf", "ncfn", "nsetups"):
+        assert st[k] == so[k], (k, st, so)
+    assert np.abs(out.cpu().numpy() - yo).max() <= 1e-6
