@@ -66,7 +66,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // The FP64 input is rounded to R on load (R = float: mixed chain).  FIX > 0:
 // the compile-time plan of that length, whose first pass reads its inputs
 // from HBM directly and, for an open-boundary row (row_len <= n/2), skips the
-// zero-padded upper half of every butterfly; FIX = 0: the runtime plan.
+// zero-padded upper half of every butterfly; FIX = 0: the runtime plan, -1:
+// the runtime plan of a length with a prime factor above 5.
 template <typename R, int NB, int EPT, int FIX>
 __global__ void k_rows_fwd(FftPlanT<R> pl, const double* __restrict__ in, long long comp_stride, int row_len,
                            int nrows, const double* __restrict__ w, cx_t<R>* __restrict__ S, int ld, int Hx) {
@@ -109,7 +110,7 @@ __global__ void k_rows_fwd(FftPlanT<R> pl, const double* __restrict__ in, long l
   } else {
     for (int i = threadIdx.x; i < n; i += blockDim.x) buf[fpad<R, true>(i)] = load_in(i);
     __syncthreads();
-    fft_stockham<R, -1, EPT, true>(buf, pl);
+    fft_stockham<R, -1, EPT, true, FIX < 0>(buf, pl);
   }
   const int T = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + threadIdx.x;
   for (int e = tid; e < Hx * 2 * NB; e += T) {
@@ -130,7 +131,7 @@ __global__ void k_rows_fwd(FftPlanT<R> pl, const double* __restrict__ in, long l
 template <typename R, int SIGN, int EPT, int FIX>
 __device__ __forceinline__ void col_fft(cx_t<R>* buf, const FftPlanT<R>& pl) {
   if constexpr (FIX > 0) fft_fixed<R, SIGN, EPT, false, FIX, 0, fixed_radices(FIX).nr, 1>(buf, pl);
-  else fft_stockham<R, SIGN, EPT>(buf, pl);
+  else fft_stockham<R, SIGN, EPT, false, FIX < 0>(buf, pl);
 }
 
 // ── K2: column transform + tensor multiply + inverse column transform ─────
@@ -351,7 +352,7 @@ __global__ void k_rows_inv(FftPlanT<R> pl, const cx_t<R>* __restrict__ S, int ld
       stockham_last_pass_st<R, RL, +1, EPT, true, false>(buf, pl, FIX, st);
     }
   } else {
-    fft_stockham<R, +1, EPT, true>(buf, pl);
+    fft_stockham<R, +1, EPT, true, FIX < 0>(buf, pl);
     const int T = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + threadIdx.x;
 #pragma unroll
     for (int r = 0; r < NB * 2; r++) {
@@ -520,7 +521,7 @@ static bool fixed_radix(int r) {
 
 struct HostFft {
   int n = 0, tx = 32, ept = 8;
-  int fix = 0;   // n when the compile-time plan runs (fixed_length), else 0
+  int fix = 0;   // n when the compile-time plan runs (fixed_length), -1 with a prime factor above 5, else 0
   std::vector<int> radix;
   double2* d_tw = nullptr;
   float2* d_twf = nullptr;   // FP32 twiddles (mixed chain)
@@ -529,7 +530,7 @@ struct HostFft {
   // fixed radices; a generic radix R needs one thread per butterfly (n/R)
   int tx_for(int e) const {
     int need = (n + e - 1) / e;
-    if (!fix)
+    if (fix <= 0)
       for (int r : radix)
         if (!fixed_radix(r)) need = std::max(need, n / r);
     return ((std::max(need, 32) + 31) / 32) * 32;
@@ -603,8 +604,10 @@ static int fft_init(HostFft& f, int n, int batch) {
     llg_set_error("FFT length " + std::to_string(n) + " has a prime factor > 64");
     return LLG_ERR_NOTSUP;
   }
+  for (int r : f.radix)
+    if (!f.fix && !fixed_radix(r)) f.fix = -1;
   // threads per transform: n/16 covers the fixed radices (<= 16/R butterflies
-  // per thread); a generic radix R needs one thread per butterfly (n/R).
+  // per thread); a generic radix R gets one thread per butterfly (n/R) at least.
   f.ept = (((n + 7) / 8 + 31) / 32 * 32 * batch <= 1024) ? 8 : 16;
   int need = (n + f.ept - 1) / f.ept;
   for (int r : f.radix)
@@ -683,6 +686,7 @@ using ColsFwdFn = void (*)(FftPlan, double2*, int, int, int);
     case 2048: return EXPR_OF(2048);                                          \
     case 3072: return EXPR_OF(3072);                                          \
     case 4096: return EXPR_OF(4096);                                          \
+    case -1: return EXPR_OF(-1);                                              \
     default: return EXPR_OF(0);                                               \
   }
 template <typename R, int NB, int EPT>

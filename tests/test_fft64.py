@@ -60,3 +60,19 @@ def test_field_matches_the_oracle(gpu, llg_lib, oracle_lib, ng, ny, opened, wind
     ctx.demag_apply(torch.from_numpy(y).to(gpu), h)
     # the chain's bound of the parity tests: device tensor and FFT against the host's
     assert rel_err(h.cpu().numpy(), want) <= 1e-11
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ng,ny,opened", [(7, 11, 0), (13, 49, 1), (61, 59, 1), (53, 3, 0), (91, 143, 0), (671, 17, 1),
+                                          (16, 1891, 0), (2, 53, 0)])
+def test_mixed_field_at_prime_lengths(gpu, llg_lib, oracle_lib, ng, ny, opened):
+    """The FP32 chain's generic passes (one output per thread; 7, 11 and 13 in
+    registers), in rows and columns, against the oracle's FP64 field."""
+    import torch
+    p = llg_lib.default_params(ng, ny, demag_mode=llg_lib.DEMAG_OPEN if opened else llg_lib.DEMAG_PERIODIC,
+                               demag_strength=2.5, demag_precision=llg_lib.DEMAG_MIXED)
+    y = np.random.default_rng(ng + ny).uniform(-1.0, 1.0, 3 * ng * ny)
+    want = oracle_lib.Oracle(p).demag(y)
+    h = torch.full((3 * ng * ny,), float("nan"), dtype=torch.float64, device=gpu)
+    llg_lib.Context(p).demag_apply(torch.from_numpy(y).to(gpu), h)
+    assert rel_err(h.cpu().numpy(), want) <= 5e-6   # the mixed chain's stated bound
