@@ -388,6 +388,7 @@ const double* llg_hdemag_device(llg_ctx* c) { return c ? c->d_hd : nullptr; }
 int llg_dot_multi(llg_ctx* c, int nvec, const double* d_x, const double* const* d_Y, double* h_out) {
   if (!c || !d_x || !d_Y || !h_out || nvec < 1 || nvec > 16) return LLG_ERR_ARG;
   const PublicReduction pr(c);
+  arm_publish(c, 8, 8 + nvec);   // the reduction's last block writes the mailbox itself
   int rc = vdot_multi_dev(c, nvec, d_x, d_Y, 8);
   if (rc) return rc;
   return fetch_scalars(c, 8, nvec, h_out);
