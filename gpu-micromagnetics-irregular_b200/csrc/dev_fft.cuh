@@ -51,6 +51,9 @@ __device__ __forceinline__ int fpad(int i) {
 }
 template <typename R>
 __host__ __device__ constexpr int padded_len(int n) { return n + (n >> (sizeof(R) == 8 ? 3 : 4)) + 1; }
+// the same rounded up to an even count (16-byte aligned data may follow)
+template <typename R>
+__host__ __device__ constexpr int padded_even(int n) { return (padded_len<R>(n) + 1) & ~1; }
 
 template <typename R>
 FFT_HD cx_t<R> cmul(cx_t<R> a, cx_t<R> b) {
