@@ -100,7 +100,19 @@ __global__ void k_rows_fwd(FftPlanT<R> pl, const double* __restrict__ in, long l
   if constexpr (FIX > 0) {
     constexpr RadixList L = fixed_radices(FIX);
     constexpr int R0 = L.r[0];
-    if constexpr (R0 % 2 == 0) {
+    // Whole rows without a window: unconditional loads, which are issued
+    // together (the general ones wait on each other's conditions, long-
+    // scoreboard 17 stall cycles per instruction).  FP32, cold L2: 2048 points,
+    // periodic 2048 rows, 82 -> 45 us; 3072 points, 512 open rows, 35 -> 22.5;
+    // 4096 points, 2048 open rows, 148 -> 92; 1024 points, 512 open, 17 -> 12.
+    const double* const pa = src + (long long)ya * row_len;
+    auto load_whole = [&](int i) -> cx_t<R> { return mk<R>((R)pa[i], (R)pa[row_len + i]); };
+    const bool whole = !w && y0 + 2 * NB <= nrows;
+    if (R0 % 2 == 0 && whole && 2 * row_len == FIX) {
+      stockham_first_pass_ld<R, R0, -1, EPT, true, R0 % 2 == 0>(buf, FIX, load_whole);
+    } else if (whole && row_len == FIX) {
+      stockham_first_pass_ld<R, R0, -1, EPT, true, false>(buf, FIX, load_whole);
+    } else if constexpr (R0 % 2 == 0) {
       if (2 * row_len <= FIX) stockham_first_pass_ld<R, R0, -1, EPT, true, true>(buf, FIX, load_in);
       else stockham_first_pass_ld<R, R0, -1, EPT, true, false>(buf, FIX, load_in);
     } else {
@@ -108,22 +120,40 @@ __global__ void k_rows_fwd(FftPlanT<R> pl, const double* __restrict__ in, long l
     }
     fft_fixed<R, -1, EPT, true, FIX, 1, L.nr, R0>(buf, pl);
   } else {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) buf[fpad<R, true>(i)] = load_in(i);
+    if (!w && y0 + 2 * NB <= nrows) {   // unconditional loads, issued together (see above)
+      const double* const pa = src + (long long)ya * row_len;
+#pragma unroll 4
+      for (int i = threadIdx.x; i < row_len; i += blockDim.x)
+        buf[fpad<R, true>(i)] = mk<R>((R)pa[i], (R)pa[row_len + i]);
+      for (int i = row_len + threadIdx.x; i < n; i += blockDim.x) buf[fpad<R, true>(i)] = mk<R>(R(0), R(0));
+    } else {
+      for (int i = threadIdx.x; i < n; i += blockDim.x) buf[fpad<R, true>(i)] = load_in(i);
+    }
     __syncthreads();
     fft_stockham<R, -1, EPT, true, FIX < 0>(buf, pl);
   }
+  // separate the two rows of every packed transform: one thread forms both
+  // (adjacent in S) of one frequency and, where the column starts allow it,
+  // stores them together
   const int T = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + threadIdx.x;
-  for (int e = tid; e < Hx * 2 * NB; e += T) {
-    const int kx = e / (2 * NB), r = e - kx * (2 * NB);
-    const int bb = r >> 1, which = r & 1;
-    const int y = y0 + r;
+  const bool pairs = (ld & 1) == 0;
+  for (int e = tid; e < Hx * NB; e += T) {
+    const int kx = e / NB, bb = e - kx * NB;
+    const int y = y0 + 2 * bb;
     if (y >= nrows) continue;
     const cx_t<R> zk = sm[bb * np + fpad<R, true>(kx)];
     const cx_t<R> zm = sm[bb * np + fpad<R, true>(kx == 0 ? 0 : n - kx)];   // (n - kx) mod n
-    cx_t<R> out;
-    if (!which) out = mk<R>(R(0.5) * (zk.x + zm.x), R(0.5) * (zk.y - zm.y));
-    else out = mk<R>(R(0.5) * (zk.y + zm.y), R(-0.5) * (zk.x - zm.x));
-    S[((long long)c * Hx + kx) * ld + y] = out;
+    const cx_t<R> oa = mk<R>(R(0.5) * (zk.x + zm.x), R(0.5) * (zk.y - zm.y));
+    const cx_t<R> ob = mk<R>(R(0.5) * (zk.y + zm.y), R(-0.5) * (zk.x - zm.x));
+    cx_t<R>* dst = &S[((long long)c * Hx + kx) * ld + y];
+    if constexpr (sizeof(R) == 4) {
+      if (pairs && y + 1 < nrows) {
+        *reinterpret_cast<float4*>(dst) = make_float4(oa.x, oa.y, ob.x, ob.y);
+        continue;
+      }
+    }
+    dst[0] = oa;
+    if (y + 1 < nrows) dst[1] = ob;
   }
 }
 
@@ -414,23 +444,34 @@ __global__ void k_rows_inv(FftPlanT<R> pl, const cx_t<R>* __restrict__ S, int ld
     constexpr int RW = 2 * NB;   // rows per column in this CTA (divides 32)
     const int T = blockDim.x * blockDim.y, tid = threadIdx.y * blockDim.x + threadIdx.x;
     const int total = Hx * RW;
-    for (int base = 0; base < total; base += T) {
-      const int e = base + tid;
-      const int kk = e / RW, r = e - kk * RW, y = y0 + r;
-      C v = mk<R>(R(0), R(0));
-      if (e < total && y < nrows) v = S[((long long)c * Hx + kk) * ld + y];
-      C w;
-      w.x = __shfl_down_sync(0xffffffffu, v.x, 1);
-      w.y = __shfl_down_sync(0xffffffffu, v.y, 1);
-      if (e < total && (r & 1) == 0) {
-        C* bp = sm + (r >> 1) * np;
-        C A = v, B = w;
-        if (kk == 0 || (even && kk == n / 2)) { A.y = R(0); B.y = R(0); }
-        bp[fpad<R, true>(kk)] = mk<R>(A.x - B.y, A.y + B.x);
-        if (kk >= 1 && kk <= n - Hx) {
-          A.y = -A.y;
-          B.y = -B.y;
-          bp[fpad<R, true>(n - kk)] = mk<R>(A.x - B.y, A.y + B.x);
+    const C* const Sc = S + (long long)c * Hx * ld + y0;
+    constexpr int LB = 4;   // loads in flight per thread (4096 points: 131 -> 94 us, 1024: 16.4 -> 14.3)
+    for (int base0 = 0; base0 < total; base0 += LB * T) {
+      C vs[LB];
+#pragma unroll
+      for (int u = 0; u < LB; u++) {
+        const int e = base0 + u * T + tid;
+        const int kk = e / RW, r = e - kk * RW;
+        vs[u] = (e < total && y0 + r < nrows) ? Sc[(long long)kk * ld + r] : mk<R>(R(0), R(0));
+      }
+#pragma unroll
+      for (int u = 0; u < LB; u++) {
+        const int e = base0 + u * T + tid;
+        const int kk = e / RW, r = e - kk * RW;
+        const C v = vs[u];
+        C w;
+        w.x = __shfl_down_sync(0xffffffffu, v.x, 1);
+        w.y = __shfl_down_sync(0xffffffffu, v.y, 1);
+        if (e < total && (r & 1) == 0) {
+          C* bp = sm + (r >> 1) * np;
+          C A = v, B = w;
+          if (kk == 0 || (even && kk == n / 2)) { A.y = R(0); B.y = R(0); }
+          bp[fpad<R, true>(kk)] = mk<R>(A.x - B.y, A.y + B.x);
+          if (kk >= 1 && kk <= n - Hx) {
+            A.y = -A.y;
+            B.y = -B.y;
+            bp[fpad<R, true>(n - kk)] = mk<R>(A.x - B.y, A.y + B.x);
+          }
         }
       }
     }
