@@ -114,7 +114,6 @@ __device__ __forceinline__ void acc_ld8(uint32_t tl, uint32_t col, float (&v)[8]
 
 template <int D1, int WPR>
 __global__ void __launch_bounds__(NT * WPR, 1) k_cols_tc(TcArgs a) {
-  pdl_entry();
   constexpr int NTW = NT * WPR;
   constexpr int K1 = 2 * D1;
   constexpr int oF1h = 0, oF1l = 128 * K1, oF2h = 256 * K1, oF2l = oF2h + 8192, oG1h = oF2h + 16384,
@@ -219,6 +218,9 @@ __global__ void __launch_bounds__(NT * WPR, 1) k_cols_tc(TcArgs a) {
     }
   };
   prefetch_group(blockIdx.x, false);
+  // everything so far is the plan's own data: it overlaps the end of the row
+  // transform, whose spectrum is first read below
+  pdl_entry();
   bool good = true;
   for (int g = blockIdx.x; g < a.ngroups && good; g += gridDim.x) {
     prefetch_group(g + gridDim.x, true);

@@ -326,6 +326,9 @@ int llg_rhs(llg_ctx* c, double t, double* d_y, double* d_ydot) {
   int rc = ready(c);
   if (rc) return rc;
   if (!d_y || !d_ydot) return LLG_ERR_ARG;
+  // up to five kernels in a row: each is launched behind the one before it
+  // (launch.h; the first waits for whatever the caller left on the stream)
+  const PdlScope pdl(c->stream == nullptr);
   rc = rhs_full(c, t, d_y, d_ydot);
   return rc ? LLG_ERR_LAUNCH : 0;
 }
@@ -369,7 +372,10 @@ int llg_demag_apply(llg_ctx* c, const double* d_y, double* d_h) {
   int rc = ready(c);
   if (rc) return rc;
   if (!d_y || !d_h) return LLG_ERR_ARG;
-  if (demag_apply(c, d_y, d_h)) return LLG_ERR_LAUNCH;
+  {
+    const PdlScope pdl(c->stream == nullptr);
+    if (demag_apply(c, d_y, d_h)) return LLG_ERR_LAUNCH;
+  }
   return demag_check(c);
 }
 
