@@ -11,6 +11,30 @@ namespace {
 constexpr int TX = 32;
 constexpr int TY = 8;
 
+// A problem whose form is known where its kernel is launched (LLG_FORMS): the
+// constants hide the members of DevProblem, so that a plain film's kernels carry
+// neither the window's loads nor the other anisotropy, and the registers they
+// cost (k_jtv_tile 58 -> 48, one more resident block: with the centre taken from
+// the tile 18.5 -> 16.3 us at 1536x512, 96 -> 78 at 2048x2048; the block inverse's
+// kernels ran slower so, 12.4 -> 14.4, and take the general problem).
+template <int WIN, int ANISO>
+struct Form : DevProblem {
+  static constexpr int windowed = WIN, aniso = ANISO;
+  Form(const DevProblem& p) : DevProblem(p) {}
+};
+// the statement with PT the Form of problem p
+#define LLG_FORMS(p, ...)                                         \
+  do {                                                            \
+    const bool cubic_ = (p).aniso == LLG_ANISO_CUBIC;             \
+    if ((p).windowed) {                                           \
+      if (cubic_) { using PT = Form<1, LLG_ANISO_CUBIC>; __VA_ARGS__; }  \
+      else { using PT = Form<1, LLG_ANISO_LINEAR>; __VA_ARGS__; }        \
+    } else {                                                      \
+      if (cubic_) { using PT = Form<0, LLG_ANISO_CUBIC>; __VA_ARGS__; }  \
+      else { using PT = Form<0, LLG_ANISO_LINEAR>; __VA_ARGS__; }        \
+    }                                                             \
+  } while (0)
+
 // Logical slot -> grid cell.  Tile slots can lie up to a tile width past the
 // edge (grids narrower than a tile), so the periodic wrap is a full modulo.
 // Periodic wrap without integer division: the tile loaders ask for indices
@@ -33,13 +57,15 @@ __device__ __forceinline__ bool map_nb(int& i, int& j, int ng, int ny, int bc) {
   return true;
 }
 
-__device__ __forceinline__ double gate_of(const DevProblem& P, int cell) {
+template <class PT>
+__device__ __forceinline__ double gate_of(const PT& P, int cell) {
   if (P.windowed) return P.w[cell];
   if (P.act) return P.act[cell] ? 1.0 : 0.0;
   return 1.0;
 }
 
-__device__ __forceinline__ void cell_axes(const DevProblem& P, int cell, double msk[3], double nsk[3]) {
+template <class PT>
+__device__ __forceinline__ void cell_axes(const PT& P, int cell, double msk[3], double nsk[3]) {
   if (P.windowed) {
     const int n = P.ncell;
     msk[0] = P.msk3[cell]; msk[1] = P.msk3[n + cell]; msk[2] = P.msk3[2 * n + cell];
@@ -50,7 +76,8 @@ __device__ __forceinline__ void cell_axes(const DevProblem& P, int cell, double 
   }
 }
 
-__device__ __forceinline__ void aniso_field(const DevProblem& P, const double m[3], const double msk[3],
+template <class PT>
+__device__ __forceinline__ void aniso_field(const PT& P, const double m[3], const double msk[3],
                                             double an[3]) {
   if (P.aniso == LLG_ANISO_CUBIC) {
 #pragma unroll
@@ -64,7 +91,8 @@ __device__ __forceinline__ void aniso_field(const DevProblem& P, const double m[
 }
 
 // symmetric local dh/dm of the anisotropy (+ window-scaled demag self term)
-__device__ __forceinline__ void aniso_jac(const DevProblem& P, const double m[3], const double msk[3],
+template <class PT>
+__device__ __forceinline__ void aniso_jac(const PT& P, const double m[3], const double msk[3],
                                           double K[3][3]) {
 #pragma unroll
   for (int a = 0; a < 3; a++)
@@ -83,7 +111,8 @@ __device__ __forceinline__ void aniso_jac(const DevProblem& P, const double m[3]
 
 // Damping of the RHS at column gi: uniform, or ramped up towards the x edges
 // in the absorbing layers (src/slit/2d_slit.cu:297-315, same expression)
-__device__ __forceinline__ double alpha_at(const DevProblem& P, int gi) {
+template <class PT>
+__device__ __forceinline__ double alpha_at(const PT& P, int gi) {
   if (P.pml_cells <= 0) return P.alpha;
   const int pml = P.pml_cells;
   double s = 0.0;
@@ -94,11 +123,13 @@ __device__ __forceinline__ double alpha_at(const DevProblem& P, int gi) {
 
 // Uniform applied field, plus the soft spin-wave source's value for the
 // current evaluation on its column (x component, src/slit/2d_slit.cu:331-349)
-__device__ __forceinline__ double happ_at(const DevProblem& P, int a, int gi) {
+template <class PT>
+__device__ __forceinline__ double happ_at(const PT& P, int a, int gi) {
   return (a == 0 && P.src_on && gi == P.src_col) ? P.happ[0] + P.src_h : P.happ[a];
 }
 
-__device__ __forceinline__ void llg_torque(const DevProblem& P, double alpha, const double m[3], const double h[3],
+template <class PT>
+__device__ __forceinline__ void llg_torque(const PT& P, double alpha, const double m[3], const double h[3],
                                            double g, double out[3]) {
   const double m1 = m[0], m2 = m[1], m3 = m[2], h1 = h[0], h2 = h[1], h3 = h[2];
   const double mh = m1 * h1 + m2 * h2 + m3 * h3;
@@ -108,7 +139,8 @@ __device__ __forceinline__ void llg_torque(const DevProblem& P, double alpha, co
 }
 
 // (I - gamma*ws*J)^-1 at frozen (m, h); closed form of 2d_i2/precond.cu:186-250
-__device__ __forceinline__ void block_inverse(const DevProblem& P, const double m[3], const double h[3],
+template <class PT>
+__device__ __forceinline__ void block_inverse(const PT& P, const double m[3], const double h[3],
                                               const double msk[3], double ws, double gamma, double Pi[9]) {
   double K[3][3];
   aniso_jac(P, m, msk, K);
@@ -175,8 +207,8 @@ struct Tile {
 
 // Stage fields f[k] (windowed: w·f) of the tile into shared memory.
 // Slot (sx, sy) holds logical cell (x0-1+sx, y0-1+sy) with the boundary rule.
-template <int NF>
-__device__ __forceinline__ void load_tile(const DevProblem& P, Tile<NF>& T, const double* const* f) {
+template <int NF, class PT>
+__device__ __forceinline__ void load_tile(const PT& P, Tile<NF>& T, const double* const* f) {
   const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
   const int tid = threadIdx.y * TX + threadIdx.x;
   const int n = P.ncell;
@@ -200,8 +232,19 @@ __device__ __forceinline__ void load_tile(const DevProblem& P, Tile<NF>& T, cons
   __syncthreads();
 }
 
+// the field's own value at this thread's cell: the staged one, or read again
+// where the tile holds the window's share of it
+template <class PT>
+__device__ __forceinline__ void tile_centre(const PT& P, const double (*F)[TY + 2][TX + 2],
+                                            const double* __restrict__ f, int cell, double m[3]) {
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+    m[a] = P.windowed ? f[a * P.ncell + cell] : F[a][threadIdx.y + 1][threadIdx.x + 1];
+}
+
 // field at a tile cell from the staged neighbours (exchange + aniso + DMI)
-__device__ __forceinline__ void tile_field(const DevProblem& P, const double (*F)[TY + 2][TX + 2],
+template <class PT>
+__device__ __forceinline__ void tile_field(const PT& P, const double (*F)[TY + 2][TX + 2],
                                            int sx, int sy, const double m[3], const double msk[3],
                                            const double nsk[3], double h[3]) {
   double an[3];
@@ -214,12 +257,14 @@ __device__ __forceinline__ void tile_field(const DevProblem& P, const double (*F
   }
 }
 
-__device__ __forceinline__ double gather_nb(const DevProblem& P, const double* f, int a, int i, int j) {
+template <class PT>
+__device__ __forceinline__ double gather_nb(const PT& P, const double* f, int a, int i, int j) {
   if (!map_nb(i, j, P.ng, P.ny, P.bc)) return 0.0;
   return f[a * P.ncell + j * P.ng + i];
 }
 
-__device__ __forceinline__ void gather_field(const DevProblem& P, const double* y, int gi, int gj,
+template <class PT>
+__device__ __forceinline__ void gather_field(const PT& P, const double* y, int gi, int gj,
                                              const double m[3], const double msk[3], const double nsk[3],
                                              double h[3]) {
   double an[3];
@@ -233,7 +278,8 @@ __device__ __forceinline__ void gather_field(const DevProblem& P, const double* 
 }
 
 // J(m)·v at one cell given field h, the staged/gathered dh pieces.
-__device__ __forceinline__ void jv_cell(const DevProblem& P, const double m[3], const double v[3],
+template <class PT>
+__device__ __forceinline__ void jv_cell(const PT& P, const double m[3], const double v[3],
                                         const double h[3], const double dh[3], double g, double o[3]) {
   const double m1 = m[0], m2 = m[1], m3 = m[2], v1 = v[0], v2 = v[1], v3 = v[2];
   const double h1 = h[0], h2 = h[1], h3 = h[2];
@@ -244,7 +290,8 @@ __device__ __forceinline__ void jv_cell(const DevProblem& P, const double m[3], 
   o[2] = g * (P.chg * (v2 * h1 + m2 * dh[0] - v1 * h2 - m1 * dh[1]) + P.alpha * (dh[2] - dmh * m3 - mh * v3));
 }
 
-__device__ __forceinline__ void dh_from(const DevProblem& P, double L, double R, double U, double D, int a,
+template <class PT>
+__device__ __forceinline__ void dh_from(const PT& P, double L, double R, double U, double D, int a,
                                         const double K[3][3], const double v[3], const double nsk[3],
                                         double& out) {
   const double kv = K[a][0] * v[0] + K[a][1] * v[1] + K[a][2] * v[2];

@@ -94,7 +94,8 @@ __global__ void k_lin_normalize(const double* __restrict__ zn0, const double* __
 
 // RHS at y with the Newton residual epilogue; writes −res (the Newton
 // iteration's negated right-hand side) and no ydot.
-__global__ void __launch_bounds__(TX * TY) k_rhs_resid_tile(DevProblem P, const double* __restrict__ y,
+template <class PT>
+__global__ void __launch_bounds__(TX * TY) k_rhs_resid_tile(PT P, const double* __restrict__ y,
                                                             const double* __restrict__ hd,
                                                             const double* __restrict__ zn1,
                                                             const double* __restrict__ ycor, double rl1,
@@ -112,7 +113,8 @@ __global__ void __launch_bounds__(TX * TY) k_rhs_resid_tile(DevProblem P, const 
   const int gi = blockIdx.x * TX + threadIdx.x, gj = blockIdx.y * TY + threadIdx.y;
   if (gi >= P.ng || gj >= P.ny) return;
   const int n = P.ncell, cell = gj * P.ng + gi;
-  const double m[3] = {y[cell], y[n + cell], y[2 * n + cell]};
+  double m[3];
+  tile_centre(P, T.v[0], y, cell, m);
   double msk[3], nsk[3];
   cell_axes(P, cell, msk, nsk);
   double h[3];
@@ -591,7 +593,8 @@ int fused_resid(llg_ctx* c, const double* y, const double* zn1, const double* yc
                                                                    gamma, negres, da);
   } else {
     dim3 g((c->p.ng + TX - 1) / TX, (c->p.ny + TY - 1) / TY);
-    klaunch(k_rhs_resid_tile, g, dim3(TX, TY), 0, c->stream, c->dp, y, c->d_hd, zn1, ycor, rl1, gamma, negres, da);
+    LLG_FORMS(c->dp, klaunch(k_rhs_resid_tile<PT>, g, dim3(TX, TY), 0, c->stream, PT(c->dp), y, c->d_hd, zn1, ycor, rl1,
+                             gamma, negres, da));
   }
   LLG_CUDA_TRY(cudaPeekAtLastError());
   return 0;
@@ -604,8 +607,8 @@ static int psolve_scale_dot_impl(llg_ctx* c, const double* r, const double* ewt,
   LLG_COUNT(KID_PSOLVE);
   const float* pinvf = (sizeof(VT) == sizeof(float) && c->pinv_f32 && !da) ? reinterpret_cast<const float*>(c->d_pinv)
                                                                           : nullptr;
-  klaunch(k_psolve_scale_dot<VT>, red_blocks(c->ncell, c->red_per), RT, 0, c->stream, c->dp, c->d_pm, c->d_ph, pinvf, r, ewt,
-          v0, c->gamma_setup, c->d_red, c->d_counter, c->d_scal + slot, da,
+  klaunch(k_psolve_scale_dot<VT>, red_blocks(c->ncell, c->red_per), RT, 0, c->stream, c->dp, c->d_pm, c->d_ph, pinvf, r,
+          ewt, v0, c->gamma_setup, c->d_red, c->d_counter, c->d_scal + slot, da,
           slot_aout >= 0 ? c->d_scal + slot_aout : nullptr);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   return 0;

@@ -55,7 +55,8 @@ __global__ void k_normalize(double* __restrict__ y, int n, int kind, double eps)
   }
 }
 
-__global__ void __launch_bounds__(TX * TY) k_rhs_tile(DevProblem P, const double* __restrict__ y,
+template <class PT>
+__global__ void __launch_bounds__(TX * TY) k_rhs_tile(PT P, const double* __restrict__ y,
                                                       const double* __restrict__ hd,
                                                       double* __restrict__ ydot) {
   pdl_entry();
@@ -65,7 +66,8 @@ __global__ void __launch_bounds__(TX * TY) k_rhs_tile(DevProblem P, const double
   const int gi = blockIdx.x * TX + threadIdx.x, gj = blockIdx.y * TY + threadIdx.y;
   if (gi >= P.ng || gj >= P.ny) return;
   const int n = P.ncell, cell = gj * P.ng + gi;
-  const double m[3] = {y[cell], y[n + cell], y[2 * n + cell]};
+  double m[3];
+  tile_centre(P, T.v[0], y, cell, m);
   double msk[3], nsk[3];
   cell_axes(P, cell, msk, nsk);
   double h[3];
@@ -103,7 +105,8 @@ __global__ void k_rhs_compact(DevProblem P, const double* __restrict__ y, const 
   }
 }
 
-__global__ void __launch_bounds__(TX * TY) k_jtv_tile(DevProblem P, const double* __restrict__ v,
+template <class PT>
+__global__ void __launch_bounds__(TX * TY) k_jtv_tile(PT P, const double* __restrict__ v,
                                                       double* __restrict__ Jv, const double* __restrict__ y,
                                                       const double* __restrict__ hd) {
   pdl_entry();
@@ -114,8 +117,9 @@ __global__ void __launch_bounds__(TX * TY) k_jtv_tile(DevProblem P, const double
   if (gi >= P.ng || gj >= P.ny) return;
   const int n = P.ncell, cell = gj * P.ng + gi;
   const int sx = threadIdx.x + 1, sy = threadIdx.y + 1;
-  const double m[3] = {y[cell], y[n + cell], y[2 * n + cell]};
-  const double vv[3] = {v[cell], v[n + cell], v[2 * n + cell]};
+  double m[3], vv[3];
+  tile_centre(P, T.v[0], y, cell, m);
+  tile_centre(P, T.v[1], v, cell, vv);
   double msk[3], nsk[3];
   cell_axes(P, cell, msk, nsk);
   double h[3];
@@ -182,7 +186,8 @@ __global__ void k_jtv_compact(DevProblem P, const double* __restrict__ v, double
 }
 
 // psetup: freeze (m, h_total) per cell
-__global__ void __launch_bounds__(TX * TY) k_psetup_tile(DevProblem P, const double* __restrict__ y,
+template <class PT>
+__global__ void __launch_bounds__(TX * TY) k_psetup_tile(PT P, const double* __restrict__ y,
                                                          const double* __restrict__ hd, double* __restrict__ pm,
                                                          double* __restrict__ ph, double* __restrict__ pinv,
                                                          double gamma, const DevArgs* da, int pinv_f32) {
@@ -195,7 +200,8 @@ __global__ void __launch_bounds__(TX * TY) k_psetup_tile(DevProblem P, const dou
   const int gi = blockIdx.x * TX + threadIdx.x, gj = blockIdx.y * TY + threadIdx.y;
   if (gi >= P.ng || gj >= P.ny) return;
   const int n = P.ncell, cell = gj * P.ng + gi;
-  const double m[3] = {y[cell], y[n + cell], y[2 * n + cell]};
+  double m[3];
+  tile_centre(P, T.v[0], y, cell, m);
   double msk[3], nsk[3];
   cell_axes(P, cell, msk, nsk);
   double h[3];
@@ -245,7 +251,7 @@ __global__ void k_psolve(DevProblem P, const double* __restrict__ pm, const doub
 // Fused Arnoldi operator of left-preconditioned, ewt-scaled GMRES:
 //   vt = in / s ;  u = vt − γ J(y) vt ;  out = s ⊙ P^-1 u
 // One pass: reads in (stencil), s (stencil), y (stencil), pm/ph, writes out.
-template <typename VT = double>
+template <typename VT>
 __global__ void __launch_bounds__(TX * TY, 4) k_arnoldi_tile(DevProblem P, const VT* __restrict__ in,
                                                           const double* __restrict__ s,
                                                           VT* __restrict__ out, const double* __restrict__ y,
@@ -384,8 +390,8 @@ __device__ __forceinline__ void ap_slot(int q, int& sx, int& sy) {
   else { const int r2 = q - (TY + 2) * TX; sy = r2 >> 1; sx = (r2 & 1) ? (TX + 1) : 0; }
 }
 
-template <typename VT = double>
-__global__ void __launch_bounds__(AP_NT, 3) k_arnoldi_pipe(DevProblem P, const VT* __restrict__ in,
+template <typename VT, class PT>
+__global__ void __launch_bounds__(AP_NT, 3) k_arnoldi_pipe(PT P, const VT* __restrict__ in,
                                                            const double* __restrict__ s,
                                                            VT* __restrict__ out, const double* __restrict__ y,
                                                            const double* __restrict__ hd,
@@ -570,7 +576,7 @@ int launch_rhs(llg_ctx* c, const double* y, const double* hd, double* ydot) {
                                                                c->d_inactive_ids, c->n_inactive);
   } else {
     LLG_COUNT(KID_RHS);
-    klaunch(k_rhs_tile, tile_grid(c), dim3(TX, TY), 0, c->stream, c->dp, y, hd, ydot);
+    LLG_FORMS(c->dp, klaunch(k_rhs_tile<PT>, tile_grid(c), dim3(TX, TY), 0, c->stream, PT(c->dp), y, hd, ydot));
   }
   LLG_CUDA_TRY(cudaPeekAtLastError());
   return 0;
@@ -590,7 +596,8 @@ int launch_jtv(llg_ctx* c, const double* v, double* Jv, const double* y) {
                                                                c->n_active, c->d_inactive_ids, c->n_inactive);
   } else {
     LLG_COUNT(KID_JTV);
-    klaunch(k_jtv_tile, tile_grid(c), dim3(TX, TY), 0, c->stream, P, v, Jv, y, c->d_hd);
+    LLG_FORMS(P, klaunch(k_jtv_tile<PT>, tile_grid(c), dim3(TX, TY), 0, c->stream, PT(P), v, Jv, y,
+                         (const double*)c->d_hd));
   }
   LLG_CUDA_TRY(cudaPeekAtLastError());
   return 0;
@@ -598,8 +605,8 @@ int launch_jtv(llg_ctx* c, const double* v, double* Jv, const double* y) {
 
 int launch_psetup(llg_ctx* c, const double* y, double gamma, const DevArgs* da) {
   LLG_COUNT(KID_PSETUP);
-  klaunch(k_psetup_tile, tile_grid(c), dim3(TX, TY), 0, c->stream, c->dp, y, c->d_hd, c->d_pm, c->d_ph, c->d_pinv,
-          gamma, da, c->pinv_f32);
+  LLG_FORMS(c->dp, klaunch(k_psetup_tile<PT>, tile_grid(c), dim3(TX, TY), 0, c->stream, PT(c->dp), y, c->d_hd, c->d_pm,
+                           c->d_ph, c->d_pinv, gamma, da, c->pinv_f32));
   LLG_CUDA_TRY(cudaPeekAtLastError());
   c->gamma_setup = gamma;
   c->have_setup = 1;
@@ -614,12 +621,13 @@ int launch_psolve(llg_ctx* c, const double* r, double* z, const DevArgs* da) {
   return 0;
 }
 
-int arnoldi_setup(llg_ctx* c) {
+template <class PT>
+static int arnoldi_setup_form(llg_ctx* c) {
   const size_t smax = 2 * sizeof(double) * ap_buf_doubles(1);
   const size_t smaxf = 2 * sizeof(double) * ap_buf_doubles(1, 1);
-  if (cudaFuncSetAttribute((const void*)k_arnoldi_pipe<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if (cudaFuncSetAttribute((const void*)k_arnoldi_pipe<double, DevProblem>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smax) != cudaSuccess ||
-      cudaFuncSetAttribute((const void*)k_arnoldi_pipe<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaFuncSetAttribute((const void*)k_arnoldi_pipe<float, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smaxf) != cudaSuccess) {
     llg_set_error("arnoldi operator: shared-memory opt-in failed");
     return LLG_ERR_CUDA;
@@ -627,9 +635,9 @@ int arnoldi_setup(llg_ctx* c) {
   const long long ntiles = (long long)((c->p.ng + TX - 1) / TX) * ((c->p.ny + TY - 1) / TY);
   for (int jf = 0; jf < 2; jf++) {
     int per_sm = 0, per_sm_f = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_arnoldi_pipe<double>, AP_NT,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_arnoldi_pipe<double, DevProblem>, AP_NT,
                                                       2 * sizeof(double) * ap_buf_doubles(jf)) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f, k_arnoldi_pipe<float>, AP_NT,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f, k_arnoldi_pipe<float, PT>, AP_NT,
                                                       2 * sizeof(double) * ap_buf_doubles(jf, 1)) != cudaSuccess ||
         per_sm < 1 || per_sm_f < 1) {
       llg_set_error("arnoldi operator: occupancy query failed");
@@ -641,6 +649,11 @@ int arnoldi_setup(llg_ctx* c) {
   return 0;
 }
 
+int arnoldi_setup(llg_ctx* c) {   // (a windowed problem runs k_arnoldi_tile, which needs none of this)
+  return c->p.aniso_kind == LLG_ANISO_CUBIC ? arnoldi_setup_form<Form<0, LLG_ANISO_CUBIC>>(c)
+                                            : arnoldi_setup_form<Form<0, LLG_ANISO_LINEAR>>(c);
+}
+
 // Autotune of the persistent operator's grid: the first launch of a (grid
 // size, staged field, basis precision) shape times the kernel at 1, 2, ...
 // CTAs per SM up to the occupancy limit on the live buffers (each candidate
@@ -648,13 +661,13 @@ int arnoldi_setup(llg_ctx* c) {
 // grid does not change any cell's arithmetic; the candidates' outputs are
 // overwritten by the launch that follows.
 static std::mutex g_arn_mu;
-static std::map<std::tuple<int, int, int, int>, int> g_arn_tuned;
+static std::map<std::tuple<int, int, int, int, int>, int> g_arn_tuned;
 
-template <typename VT>
-static int arnoldi_tune(llg_ctx* c, const DevProblem& P, int jf, const VT* in, const double* ewt, VT* out,
+template <typename VT, class PT>
+static int arnoldi_tune(llg_ctx* c, const PT& P, int jf, const VT* in, const double* ewt, VT* out,
                         const double* y, double gamma, int scale_out, const double* in_a, int* grid) {
   constexpr int f32 = sizeof(VT) != sizeof(double) ? 1 : 0;
-  const auto key = std::make_tuple(c->p.ng, c->p.ny, jf, f32);
+  const auto key = std::make_tuple(c->p.ng, c->p.ny, jf, f32, (int)c->p.aniso_kind);
   {
     std::lock_guard<std::mutex> g(g_arn_mu);
     auto it = g_arn_tuned.find(key);
@@ -673,7 +686,7 @@ static int arnoldi_tune(llg_ctx* c, const DevProblem& P, int jf, const VT* in, c
     float ms = 0.f;
     for (int rep = 0; rep < 2; rep++) {
       cudaEventRecord(e0, c->stream);
-      k_arnoldi_pipe<VT><<<gsz, AP_NT, smem, c->stream>>>(P, in, ewt, out, y, c->d_hd,
+      k_arnoldi_pipe<VT, PT><<<gsz, AP_NT, smem, c->stream>>>(P, in, ewt, out, y, c->d_hd,
                                                           reinterpret_cast<const VT*>(c->d_pinv), gamma, scale_out,
                                                           nullptr, in_a);
       cudaEventRecord(e1, c->stream);
@@ -695,6 +708,16 @@ static int arnoldi_tune(llg_ctx* c, const DevProblem& P, int jf, const VT* in, c
   g_arn_tuned[key] = best;
   return 0;
 }
+
+// the statement with PT the problem type of k_arnoldi_pipe<VT>: the FP32 basis's
+// kernel gains from a known form (1536x512: 30.1 -> 28.3 us), the FP64 one spills
+// more (35.8 -> 36.8) and takes the general problem
+#define PIPE_FORM(...)                                                                        \
+  do {                                                                                        \
+    if constexpr (sizeof(VT) == sizeof(double)) { using PT = DevProblem; __VA_ARGS__; }       \
+    else if (P.aniso == LLG_ANISO_CUBIC) { using PT = Form<0, LLG_ANISO_CUBIC>; __VA_ARGS__; } \
+    else { using PT = Form<0, LLG_ANISO_LINEAR>; __VA_ARGS__; }                               \
+  } while (0)
 
 template <typename VT>
 static int arnoldi_op_impl(llg_ctx* c, const VT* in, const double* ewt, VT* out, const double* y, double gamma,
@@ -718,20 +741,22 @@ static int arnoldi_op_impl(llg_ctx* c, const VT* in, const double* ewt, VT* out,
   }
   LLG_COUNT(KID_ARNOLDI);
   ktimer_mark(c, KID_ARNOLDI, true);
+  const VT* const pinv = reinterpret_cast<const VT*>(c->d_pinv);
+  const double* const hd = c->d_hd;
   if (c->dp.windowed) {
-    klaunch(k_arnoldi_tile<VT>, tile_grid(c), dim3(TX, TY), 0, c->stream, P, in, ewt, out, y, c->d_hd,
-            reinterpret_cast<const VT*>(c->d_pinv), gamma, scale_out, da, in_a);
+    klaunch(k_arnoldi_tile<VT>, tile_grid(c), dim3(TX, TY), 0, c->stream, P, in, ewt, out, y, hd, pinv, gamma, scale_out,
+            da, in_a);
   } else {
     const int jf = c->dp.jv_full ? 1 : 0;
     int& grid = f32 ? c->arn_grid_f[jf] : c->arn_grid[jf];
     if (!da && !c->capturing && !(f32 ? c->arn_tuned_f[jf] : c->arn_tuned[jf])) {
-      const int rc = arnoldi_tune<VT>(c, P, jf, in, ewt, out, y, gamma, scale_out, in_a, &grid);
+      int rc = 0;
+      PIPE_FORM(rc = (arnoldi_tune<VT, PT>(c, PT(P), jf, in, ewt, out, y, gamma, scale_out, in_a, &grid)));
       if (rc) return rc;
       (f32 ? c->arn_tuned_f[jf] : c->arn_tuned[jf]) = 1;
     }
-    klaunch(k_arnoldi_pipe<VT>, grid, AP_NT,
-            2 * sizeof(double) * ap_buf_doubles(jf, f32), c->stream, P, in, ewt, out, y, c->d_hd,
-            reinterpret_cast<const VT*>(c->d_pinv), gamma, scale_out, da, in_a);
+    PIPE_FORM(klaunch(k_arnoldi_pipe<VT, PT>, grid, AP_NT, 2 * sizeof(double) * ap_buf_doubles(jf, f32), c->stream,
+                      PT(P), in, ewt, out, y, hd, pinv, gamma, scale_out, da, in_a));
   }
   ktimer_mark(c, KID_ARNOLDI, false);
   LLG_CUDA_TRY(cudaPeekAtLastError());
