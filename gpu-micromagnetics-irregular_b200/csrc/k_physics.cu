@@ -79,18 +79,38 @@ __global__ void __launch_bounds__(TX * TY) k_rhs_tile(PT P, const double* __rest
   ydot[cell] = o[0]; ydot[n + cell] = o[1]; ydot[2 * n + cell] = o[2];
 }
 
-__global__ void k_rhs_compact(DevProblem P, const double* __restrict__ y, const double* __restrict__ hd,
+// Zeros to the listed cells of a field: four ids of a thread's slice are read
+// together, so that the stores do not wait on one id after another.
+__device__ __forceinline__ void zero_listed(double* __restrict__ f, int n, const int32_t* __restrict__ ids, int ni) {
+  const int st = gridDim.x * blockDim.x;
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  for (; t < ni - 3 * st; t += 4 * st) {
+    int cell[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) cell[u] = ids[t + u * st];
+#pragma unroll
+    for (int u = 0; u < 4; u++) { f[cell[u]] = 0.0; f[n + cell[u]] = 0.0; f[2 * n + cell[u]] = 0.0; }
+  }
+  for (; t < ni; t += st) {
+    const int cell = ids[t];
+    f[cell] = 0.0; f[n + cell] = 0.0; f[2 * n + cell] = 0.0;
+  }
+}
+
+// Active cells first, the next one's id read ahead of the current one's
+// stencil; then zeros to the inactive ones.  2048x2048, active circle of radius
+// N/4: 44 -> 40 us.
+template <class PT>
+__global__ void k_rhs_compact(PT P, const double* __restrict__ y, const double* __restrict__ hd,
                               double* __restrict__ ydot, const int32_t* __restrict__ act_ids, int na,
                               const int32_t* __restrict__ inact_ids, int ni) {
   pdl_entry();
-  const int n = P.ncell;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < na + ni; t += gridDim.x * blockDim.x) {
-    if (t >= na) {
-      const int cell = inact_ids[t - na];
-      ydot[cell] = 0.0; ydot[n + cell] = 0.0; ydot[2 * n + cell] = 0.0;
-      continue;
-    }
-    const int cell = act_ids[t];
+  const int n = P.ncell, st = gridDim.x * blockDim.x;
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  int next = t < na ? act_ids[t] : 0;
+  for (; t < na; t += st) {
+    const int cell = next;
+    if (t < na - st) next = act_ids[t + st];
     const int gi = cell % P.ng, gj = cell / P.ng;
     const double m[3] = {y[cell], y[n + cell], y[2 * n + cell]};
     double msk[3], nsk[3];
@@ -103,6 +123,7 @@ __global__ void k_rhs_compact(DevProblem P, const double* __restrict__ y, const 
     llg_torque(P, alpha_at(P, gi), m, h, 1.0, o);
     ydot[cell] = o[0]; ydot[n + cell] = o[1]; ydot[2 * n + cell] = o[2];
   }
+  zero_listed(ydot, n, inact_ids, ni);
 }
 
 template <class PT>
@@ -144,19 +165,18 @@ __global__ void __launch_bounds__(TX * TY) k_jtv_tile(PT P, const double* __rest
   Jv[cell] = o[0]; Jv[n + cell] = o[1]; Jv[2 * n + cell] = o[2];
 }
 
-__global__ void k_jtv_compact(DevProblem P, const double* __restrict__ v, double* __restrict__ Jv,
+template <class PT>
+__global__ void k_jtv_compact(PT P, const double* __restrict__ v, double* __restrict__ Jv,
                               const double* __restrict__ y, const double* __restrict__ hd,
                               const int32_t* __restrict__ act_ids, int na, const int32_t* __restrict__ inact_ids,
                               int ni) {
   pdl_entry();
-  const int n = P.ncell;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < na + ni; t += gridDim.x * blockDim.x) {
-    if (t >= na) {
-      const int cell = inact_ids[t - na];
-      Jv[cell] = 0.0; Jv[n + cell] = 0.0; Jv[2 * n + cell] = 0.0;
-      continue;
-    }
-    const int cell = act_ids[t];
+  const int n = P.ncell, st = gridDim.x * blockDim.x;
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  int next = t < na ? act_ids[t] : 0;
+  for (; t < na; t += st) {
+    const int cell = next;
+    if (t < na - st) next = act_ids[t + st];
     const int gi = cell % P.ng, gj = cell / P.ng;
     const double m[3] = {y[cell], y[n + cell], y[2 * n + cell]};
     const double vv[3] = {v[cell], v[n + cell], v[2 * n + cell]};
@@ -183,6 +203,7 @@ __global__ void k_jtv_compact(DevProblem P, const double* __restrict__ v, double
     jv_cell(P, m, vv, h, dh, 1.0, o);
     Jv[cell] = o[0]; Jv[n + cell] = o[1]; Jv[2 * n + cell] = o[2];
   }
+  zero_listed(Jv, n, inact_ids, ni);
 }
 
 // psetup: freeze (m, h_total) per cell
@@ -572,8 +593,9 @@ int launch_rhs(llg_ctx* c, const double* y, const double* hd, double* ydot) {
   if (c->p.exec_model == LLG_EXEC_COMPACT) {
     const int tot = c->n_active + c->n_inactive;
     LLG_COUNT(KID_RHS);
-    klaunch(k_rhs_compact, grid_1d(c, tot, 256), 256, 0, c->stream, c->dp, y, hd, ydot, c->d_active_ids, c->n_active,
-                                                               c->d_inactive_ids, c->n_inactive);
+    LLG_FORMS(c->dp, klaunch(k_rhs_compact<PT>, grid_1d(c, tot, 256), 256, 0, c->stream, PT(c->dp), y, hd, ydot,
+                             (const int32_t*)c->d_active_ids, c->n_active, (const int32_t*)c->d_inactive_ids,
+                             c->n_inactive));
   } else {
     LLG_COUNT(KID_RHS);
     LLG_FORMS(c->dp, klaunch(k_rhs_tile<PT>, tile_grid(c), dim3(TX, TY), 0, c->stream, PT(c->dp), y, hd, ydot));
@@ -592,8 +614,9 @@ int launch_jtv(llg_ctx* c, const double* v, double* Jv, const double* y) {
   if (c->p.exec_model == LLG_EXEC_COMPACT) {
     const int tot = c->n_active + c->n_inactive;
     LLG_COUNT(KID_JTV);
-    klaunch(k_jtv_compact, grid_1d(c, tot, 256), 256, 0, c->stream, P, v, Jv, y, c->d_hd, c->d_active_ids,
-                                                               c->n_active, c->d_inactive_ids, c->n_inactive);
+    LLG_FORMS(P, klaunch(k_jtv_compact<PT>, grid_1d(c, tot, 256), 256, 0, c->stream, PT(P), v, Jv, y,
+                         (const double*)c->d_hd, (const int32_t*)c->d_active_ids, c->n_active,
+                         (const int32_t*)c->d_inactive_ids, c->n_inactive));
   } else {
     LLG_COUNT(KID_JTV);
     LLG_FORMS(P, klaunch(k_jtv_tile<PT>, tile_grid(c), dim3(TX, TY), 0, c->stream, PT(P), v, Jv, y,
