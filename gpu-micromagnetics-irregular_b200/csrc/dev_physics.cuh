@@ -15,8 +15,10 @@ constexpr int TY = 8;
 // constants hide the members of DevProblem, so that a plain film's kernels carry
 // neither the window's loads nor the other anisotropy, and the registers they
 // cost (k_jtv_tile 58 -> 48, one more resident block: with the centre taken from
-// the tile 18.5 -> 16.3 us at 1536x512, 96 -> 78 at 2048x2048; the block inverse's
-// kernels ran slower so, 12.4 -> 14.4, and take the general problem).
+// the tile 18.5 -> 16.3 us at 1536x512, 96 -> 78 at 2048x2048).  The kernels with
+// the block inverse take the general problem: those that apply it ran slower per
+// form, 12.4 -> 14.4, and the one that stores it rounded differently
+// (k_psetup_tile).
 template <int WIN, int ANISO>
 struct Form : DevProblem {
   static constexpr int windowed = WIN, aniso = ANISO;

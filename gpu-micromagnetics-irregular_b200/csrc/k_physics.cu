@@ -206,9 +206,12 @@ __global__ void k_jtv_compact(PT P, const double* __restrict__ v, double* __rest
   zero_listed(Jv, n, inact_ids, ni);
 }
 
-// psetup: freeze (m, h_total) per cell
-template <class PT>
-__global__ void __launch_bounds__(TX * TY) k_psetup_tile(PT P, const double* __restrict__ y,
+// psetup: freeze (m, h_total) per cell.  The general problem in every form:
+// with the form known, the compiler contracts the block inverse's products
+// differently (a windowed or cubic film's stored inverse then differs in
+// 0.01..3 % of its entries from the one k_psolve forms), and the FP32 parts of
+// a mixed film amplify that.
+__global__ void __launch_bounds__(TX * TY) k_psetup_tile(DevProblem P, const double* __restrict__ y,
                                                          const double* __restrict__ hd, double* __restrict__ pm,
                                                          double* __restrict__ ph, double* __restrict__ pinv,
                                                          double gamma, const DevArgs* da, int pinv_f32) {
@@ -628,8 +631,8 @@ int launch_jtv(llg_ctx* c, const double* v, double* Jv, const double* y) {
 
 int launch_psetup(llg_ctx* c, const double* y, double gamma, const DevArgs* da) {
   LLG_COUNT(KID_PSETUP);
-  LLG_FORMS(c->dp, klaunch(k_psetup_tile<PT>, tile_grid(c), dim3(TX, TY), 0, c->stream, PT(c->dp), y, c->d_hd, c->d_pm,
-                           c->d_ph, c->d_pinv, gamma, da, c->pinv_f32));
+  klaunch(k_psetup_tile, tile_grid(c), dim3(TX, TY), 0, c->stream, c->dp, y, c->d_hd, c->d_pm, c->d_ph, c->d_pinv,
+          gamma, da, c->pinv_f32);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   c->gamma_setup = gamma;
   c->have_setup = 1;
