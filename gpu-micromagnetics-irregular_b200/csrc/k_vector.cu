@@ -196,7 +196,9 @@ __global__ void k_lincomb(int nv, CoefPack c, PtrPack X, double* z, long long n)
 }
 // the same with the vector count fixed at compile time: the loads of all NV
 // vectors for four slice elements are issued before any of them is used
-// (1536x512: 2 vectors, 57 MB, 15.5 -> 9.3 us; 4 vectors, 94 MB, 14.6 us)
+// (1536x512: 2 vectors, 57 MB, 15.5 -> 9.3 us; 4 vectors, 94 MB, 14.6 us).  The
+// fma is written out: of an unrolled sum the compiler may round c1 x1 and fuse
+// c0 x0 instead, another last bit than k_lincomb's.
 template <int NV>
 __global__ void __launch_bounds__(256) k_lincomb_k(CoefPack c, PtrPack X, double* z, long long n) {
   pdl_entry();
@@ -211,7 +213,7 @@ __global__ void __launch_bounds__(256) k_lincomb_k(CoefPack c, PtrPack X, double
     for (int u = 0; u < UB; u++) {
       double s = c.c[0] * x[u][0];
 #pragma unroll
-      for (int k = 1; k < NV; k++) s = c.c[k] * x[u][k] + s;
+      for (int k = 1; k < NV; k++) s = fma(c.c[k], x[u][k], s);
       if (i0 + u * st < n) z[i0 + u * st] = s;
     }
   }
