@@ -452,7 +452,7 @@ __global__ void k_rows_inv(FftPlanT<R> pl, const cx_t<R>* __restrict__ S, int ld
       for (int u = 0; u < LB; u++) {
         const int e = base0 + u * T + tid;
         const int kk = e / RW, r = e - kk * RW;
-        vs[u] = (e < total && y0 + r < nrows) ? Sc[(long long)kk * ld + r] : mk<R>(R(0), R(0));
+        vs[u] = (e < total && y0 + r < nrows) ? __ldcg(&Sc[(long long)kk * ld + r]) : mk<R>(R(0), R(0));   // (launch.h)
       }
 #pragma unroll
       for (int u = 0; u < LB; u++) {

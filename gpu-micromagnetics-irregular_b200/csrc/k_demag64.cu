@@ -51,15 +51,16 @@ __device__ __forceinline__ d4 ldg4(const d4* p) {   // 32 bytes, read-only data
   asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
   return v;
 }
+// (past L1: the column kernel before it rewrote S in place, see launch.h)
 __device__ __forceinline__ void ld2(const dcx* p, bool vec, bool both, dcx& a, dcx& b) {
   if (vec && both) {
-    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.cg.v4.f64 {%0, %1, %2, %3}, [%4];"
                  : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y)
                  : "l"(p)
                  : "memory");
   } else {
-    a = p[0];
-    b = both ? p[1] : mk<double>(0.0, 0.0);
+    a = __ldcg(p);
+    b = both ? __ldcg(p + 1) : mk<double>(0.0, 0.0);
   }
 }
 __device__ __forceinline__ void st2(dcx* p, bool vec, bool both, dcx a, dcx b) {

@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(RT) k_predict_fused(ZPack zn, CPack f, int pen
 #pragma unroll
     for (int a = 0; a < 3; a++)
 #pragma unroll
-      for (int j = 0; j <= Q; j++) v[a][j] = zn.p[j][(long long)a * n + cell];
+      for (int j = 0; j <= Q; j++) v[a][j] = __ldcg(&zn.p[j][(long long)a * n + cell]);   // (in place: launch.h)
     double xc[3] = {0.0, 0.0, 0.0};
     if (lazy) {
 #pragma unroll

@@ -40,10 +40,11 @@
 namespace {
 
 // ── kernels ────────────────────────────────────────────────────────────
+// (in place, so it reads past L1: launch.h)
 __global__ void k_normalize(double* __restrict__ y, int n, int kind, double eps) {
   pdl_entry();
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const double m1 = y[k], m2 = y[n + k], m3 = y[2 * n + k];
+    const double m1 = __ldcg(&y[k]), m2 = __ldcg(&y[n + k]), m3 = __ldcg(&y[2 * n + k]);
     const double ymp = sqrt(m1 * m1 + m2 * m2 + m3 * m3);
     if (kind == LLG_NORM_REG) {
       const double inv = 1.0 / (ymp + eps);

@@ -259,7 +259,7 @@ __global__ void k_scale_cols(int q, CoefPack f, MPtrPack zn, long long n) {
 // k_lincomb_norm with coefficients {1, -dots_0, ..., -dots_{k-1}})
 // (VT float: the stored, rounded values are what the norm sums)
 template <typename VT = double>
-__global__ void __launch_bounds__(RT) k_gs_update(int k, VPack<VT> X, const double* __restrict__ dots, VT* z,
+__global__ void __launch_bounds__(RT) k_gs_update(int k, VPack<VT> X, const double* dots, VT* z,
                                                   long long n, double* partials, unsigned int* counter,
                                                   double* out, KScale ks, double* aout, Pub pub) {
   pdl_entry();
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(RT) k_gs_update(int k, VPack<VT> X, const doub
   __syncthreads();
   double cf[MAXV - 1];
 #pragma unroll
-  for (int j = 0; j < MAXV - 1; j++) cf[j] = (j < k) ? -dots[j] : 0.0;
+  for (int j = 0; j < MAXV - 1; j++) cf[j] = (j < k) ? -slot_value(dots + j) : 0.0;
   double acc[1] = {0.0};
   const long long st = (long long)gridDim.x * RT;
   for (long long i0 = blockIdx.x * (long long)RT + threadIdx.x; i0 < n; i0 += UB * st) {
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(RT) k_gs_update(int k, VPack<VT> X, const doub
 // that of k_gs_update; it runs on one resident wave of blocks
 // (red_blocks_resident), so its sum of squares is added in another partition.
 template <int K, typename VT>
-__global__ void __launch_bounds__(RT) k_gs_update_k(VPack<VT> X, const double* __restrict__ dots, VT* z, long long n,
+__global__ void __launch_bounds__(RT) k_gs_update_k(VPack<VT> X, const double* dots, VT* z, long long n,
                                                     double* partials, unsigned int* counter, double* out, KScale ks,
                                                     double* aout, Pub pub) {
   pdl_entry();
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(RT) k_gs_update_k(VPack<VT> X, const double* _
   double cf[K], xa[K];
 #pragma unroll
   for (int j = 0; j < K; j++) {
-    cf[j] = -dots[j];
+    cf[j] = -slot_value(dots + j);
     xa[j] = xs[j];
   }
   double acc[1] = {0.0};
@@ -362,13 +362,13 @@ __global__ void __launch_bounds__(RT) k_gs_update_k(VPack<VT> X, const double* _
 // last step (Y null), z z.  Per element and per product the operations of the
 // separate pass and dot product, without the read-back between them.
 __global__ void __launch_bounds__(RT) k_mgs_step(const double* __restrict__ X, const double* xa_p,
-                                                 const double* __restrict__ hd, const double* __restrict__ Y,
+                                                 const double* hd, const double* __restrict__ Y,
                                                  const double* ya_p, double* z, long long n, double* partials,
                                                  unsigned int* counter, double* out, const double* vk, double* aout,
                                                  Pub pub) {
   pdl_entry();
   __shared__ double sm[RT / 32];
-  const double h = *hd, xa = kscale_of(xa_p), ya = kscale_of(ya_p);
+  const double h = slot_value(hd), xa = kscale_of(xa_p), ya = kscale_of(ya_p);
   double acc[1] = {0.0};
   const long long st = (long long)gridDim.x * RT;
   for (long long i0 = blockIdx.x * (long long)RT + threadIdx.x; i0 < n; i0 += UB * st) {
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(RT) k_mgs_step(const double* __restrict__ X, c
   }
   block_sum<1>(acc, sm);
   const bool last = finalize<1>(partials, gridDim.x, counter, out, 0, 1.0, acc);
-  if (last && aout && threadIdx.x == 0) *aout = mgs_scale_of(out[0], *vk);
+  if (last && aout && threadIdx.x == 0) *aout = mgs_scale_of(out[0], slot_value(vk));
   if (last) publish_carried(pub);
 }
 

@@ -16,6 +16,17 @@
 // pointers compile to.  Waiting first means a kernel is dispatched only after
 // every kernel two places before it in the stream has finished.
 //
+// That leaves the kernel just before.  C's SMs may keep a line that B loaded
+// after C was dispatched and that another block of B then rewrote: B works in
+// place, and its blocks' shares meet inside a 32-byte sector (components of an
+// odd number of cells, spectrum columns of an odd height, scalar slots next to
+// one another).  griddepcontrol.wait covers ordinary loads, not the non-coherent
+// path, so such data is read past L1 (__ldcg) on one side at least: by the
+// in-place kernels whose shares can meet so (k_normalize, k_predict_fused), by
+// the readers of the spectrum (k_rows_inv, k_rows_inv64), and in every load of a
+// scalar slot (slot_value).  The other in-place kernels' blocks own whole
+// 256-element slices of vectors that start on 256 bytes.
+//
 // A PDL launch relaxes the dependency on the preceding kernel only, so it is
 // used only where every operation of the stream between two such kernels is
 // itself a kernel: inside the host integrator's step loop on the legacy
