@@ -1,0 +1,31 @@
+"""Transform lengths with a prime factor above 5 that need many threads: the
+plan is made (its set-up kernels transform the tensor in FP64 for both forms)
+and its field is the oracle's.
+
+Lengths: 7-smooth rows and columns from 1792 points on, where a seventh of the
+length is more than 256 threads; heights above 1024 points, whose set-up takes an
+eighth of the length; the longest columns a prime factor leaves within the
+thread limits; a length whose three columns of threads pass 768."""
+import numpy as np
+import pytest
+
+import llg
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ng,ny,opened", [(1050, 6, 1), (903, 7, 1), (1400, 8, 1), (8, 910, 1), (6, 1008, 1), (5, 1040, 1),
+                                          (4, 1025, 1), (7, 2016, 0), (3, 2057, 0), (5, 2816, 0), (4, 3328, 0), (3584, 4, 0),
+                                          (5369, 3, 0), (490, 980, 0)])
+@pytest.mark.parametrize("precision", [llg.DEMAG_FP64, llg.DEMAG_MIXED])
+def test_field_matches_the_oracle(gpu, oracle_lib, ng, ny, opened, precision):
+    import torch
+    p = llg.default_params(ng, ny, demag_mode=llg.DEMAG_OPEN if opened else llg.DEMAG_PERIODIC, demag_strength=2.5,
+                           demag_precision=precision)
+    y = np.random.default_rng(ng + ny).uniform(-1.0, 1.0, 3 * ng * ny)
+    want = oracle_lib.Oracle(p).demag(y)
+    h = torch.full((3 * ng * ny,), float("nan"), dtype=torch.float64, device=gpu)
+    llg.Context(p).demag_apply(torch.from_numpy(y).to(gpu), h)
+    # the bounds of the two chains' other field tests
+    assert rel_err(h.cpu().numpy(), want) <= (1e-11 if precision == llg.DEMAG_FP64 else 5e-6)
