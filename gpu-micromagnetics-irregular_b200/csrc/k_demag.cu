@@ -723,6 +723,7 @@ struct DemagPlan {
   float* d_tzzf = nullptr;
   float2* d_txyf = nullptr;
   LaunchCfg rows, cols;          // launch shapes of the FP32 chain (autotuned)
+  int carveout = -1;             // of its launches (CarveoutScope)
   int init_ept = 8;              // elements per thread of the FP64 row transform that builds the tensor spectra
   Demag64* f64 = nullptr;        // FP64 chain (k_demag64.cu); null in the mixed form
   int* d_err = nullptr;          // wait-ran-out flag of the tensor-core column stage (the context's SLOT_TCERR)
@@ -1088,6 +1089,7 @@ static int demag_autotune(llg_ctx* c, DemagPlan* d, cx_t<R>* S, const R* txx, co
     }
   }
   cudaStream_t s = c->stream;
+  const CarveoutScope carve(d->carveout);
   const long long cs = (long long)c->ncell;
   cudaEvent_t e0, e1;
   LLG_CUDA_TRY(cudaEventCreate(&e0));
@@ -1269,6 +1271,12 @@ int demag_create(llg_ctx* c) {
     LLG_CUDA_TRY(cudaPeekAtLastError());
     // tensor-core column stage where the column shape allows it (else FP32 Stockham columns)
     rc = demag_tc_create(c, d->px, d->py, d->hx, d->ny, d->d_txxf, d->d_tyyf, d->d_tzzf, d->d_txyf, &d->tc);
+    // A narrow grid's kernels are shorter than a new split of the SMs, which
+    // chained launches ran into at every kernel: one split for the three (field
+    // of 32x512 periodic, calls back to back: 23 -> 14.5 us, 64x512 22.5 -> 15.7;
+    // on wider grids the L1 that this takes from the rows costs more,
+    // 2048x2048 396 -> 429 us)
+    if (!d->tc && 2 * d->hx <= c->num_sms) d->carveout = 100;
     if (!rc)
       rc = demag_autotune<float>(c, d, d->d_Sf, d->d_txxf, d->d_tyyf, d->d_tzzf, d->d_txyf, d->tc == nullptr);
   } else {
@@ -1286,6 +1294,7 @@ static int demag_run_stage_raw(llg_ctx* c, DemagPlan* d, int stage, const double
   const long long cs = (long long)c->ncell;
   LLG_COUNT(stage == 0 ? KID_DEMAG_ROWS_FWD : stage == 1 ? KID_DEMAG_COLS : KID_DEMAG_ROWS_INV);
   if (d->f64) return demag64_stage(c, d->f64, stage, y, w, h);
+  const CarveoutScope carve(d->carveout);
   if (stage == 0) return launch_rows_fwd<float>(d, c->stream, y, cs, d->ng, d->ny, w, d->d_Sf, d->ny, 3, d->rows);
   if (stage == 1) {
     if (d->tc) return demag_tc_cols(c, d->tc, d->d_Sf);

@@ -52,14 +52,25 @@ struct PdlScope {
 };
 inline void pdl_break() { g_pdl_break = 1; }
 
+// Shared memory's share of an SM's L1, in percent, for the launches of a scope
+// (-1: the driver's choice per kernel).  Kernels that follow one another with
+// different shares wait for the SM to drain and be split anew.
+extern thread_local int g_carveout;
+struct CarveoutScope {
+  int saved;
+  explicit CarveoutScope(int percent) : saved(g_carveout) { g_carveout = percent; }
+  ~CarveoutScope() { g_carveout = saved; }
+};
+
 template <typename... KArgs, typename... Args>
 inline void klaunch(void (*kernel)(KArgs...), dim3 g, dim3 b, size_t smem, cudaStream_t s, Args... args) {
 #ifdef LLG_PLAIN_LAUNCH
-  if (true) {
+  const bool plain = true;
 #else
-  if (g_no_pdl || g_pdl_break) {
+  const bool plain = g_no_pdl || g_pdl_break;
 #endif
-    g_pdl_break = 0;
+  if (plain) g_pdl_break = 0;
+  if (plain && g_carveout < 0) {
     kernel<<<g, b, smem, s>>>(args...);
     return;
   }
@@ -68,11 +79,18 @@ inline void klaunch(void (*kernel)(KArgs...), dim3 g, dim3 b, size_t smem, cudaS
   cfg.blockDim = b;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (!plain) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (g_carveout >= 0) {
+    at[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at[n++].val.sharedMemCarveout = (unsigned)g_carveout;
+  }
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = n;
   (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 

@@ -23,6 +23,7 @@ thread_local int g_count_off = 0;
 // integrator's step loop on the legacy default stream (PdlScope)
 thread_local int g_no_pdl = 1;
 thread_local int g_pdl_break = 0;
+thread_local int g_carveout = -1;
 int integrator_time_kernel(llg_ctx* c, int kid, int iters, double* avg_ms);
 
 int integrator_create(llg_ctx* c, double t0, const double* y0, const llg_solver_opts* o);
