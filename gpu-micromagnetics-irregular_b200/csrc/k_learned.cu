@@ -42,7 +42,7 @@ constexpr int NWT = NW1 + NW2 + NW3;   // 4032
 constexpr int TW = 32, TH = 8;         // conv tile (threads)
 constexpr int BORDER = 3;
 
-// ── convolution kernels (grid: x tiles, y tiles, batch x parts; block 32 x 8) ──
+// ── convolution kernels (grid: x tiles x parts, y tiles, batch; block 32 x 8) ──
 // A training batch is small (16 patches of 32x32: 64 tiles), so the work of a
 // tile is split over blocks as well: eight output channels each in the two
 // data passes, one tap row each in the weight gradient.  Weights are staged
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(TW * TH) k_conv3(const float* __restrict__ in,
   constexpr int PARTS = conv_parts(COUT), CO = COUT / PARTS;
   __shared__ __align__(16) float sw[CIN * 9 * CO];   // [c][t][o]
   __shared__ float st[CIN][TH + 2][TW + 2];
-  const int b = blockIdx.z / PARTS, o0 = (blockIdx.z % PARTS) * CO, x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
+  const int b = blockIdx.z, o0 = (blockIdx.x % PARTS) * CO, x0 = (blockIdx.x / PARTS) * TW, y0 = blockIdx.y * TH;
   const int tid = threadIdx.y * TW + threadIdx.x;
   const size_t plane = (size_t)H * W;
   for (int i = tid; i < CIN * 9 * CO; i += TW * TH) sw[i] = w[((o0 + i % CO) * CIN) * 9 + i / CO];
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(TW * TH) k_conv3_bwd_data(const float* __restr
   constexpr int PARTS = conv_parts(CIN), CI = CIN / PARTS;
   __shared__ __align__(16) float sw[COUT * 9 * CI];   // [o][t][c]
   __shared__ float sd[COUT][TH + 2][TW + 2];
-  const int b = blockIdx.z / PARTS, c0 = (blockIdx.z % PARTS) * CI, x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
+  const int b = blockIdx.z, c0 = (blockIdx.x % PARTS) * CI, x0 = (blockIdx.x / PARTS) * TW, y0 = blockIdx.y * TH;
   const int tid = threadIdx.y * TW + threadIdx.x;
   const size_t plane = (size_t)H * W;
   for (int i = tid; i < COUT * 9 * CI; i += TW * TH) {
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(TW * TH) k_conv3_bwd_w(const float* __restrict
   static_assert(SI % 2 == 1 && SO % 2 == 1, "odd strides");
   __shared__ float st[CIN * SI];
   __shared__ float sd[COUT * SO];
-  const int b = blockIdx.z / 3, dy = blockIdx.z % 3, x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
+  const int b = blockIdx.z, dy = blockIdx.x % 3, x0 = (blockIdx.x / 3) * TW, y0 = blockIdx.y * TH;
   const int tid = threadIdx.y * TW + threadIdx.x;
   const size_t plane = (size_t)H * W;
   const float* si = in + (size_t)b * CIN * plane;
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(TW * TH) k_conv3_bwd_w(const float* __restrict
   }
   __syncthreads();
   if (tid >= CIN * COUT) return;
-  const size_t blk = ((size_t)b * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  const size_t blk = ((size_t)b * gridDim.y + blockIdx.y) * (gridDim.x / 3) + blockIdx.x / 3;
   const float* pi = &st[(tid % CIN) * SI];
   const float* po = &sd[(tid / CIN) * SO];
   float a0 = 0.f, a1 = 0.f, a2 = 0.f;
@@ -352,7 +352,8 @@ __global__ void k_round_bf16(const float* __restrict__ w, float* __restrict__ wq
   if (i < n) wq[i] = __bfloat162float(__float2bfloat16_rn(w[i]));
 }
 
-dim3 conv_grid(int H, int W, int B, int parts = 1) { return dim3((W + TW - 1) / TW, (H + TH - 1) / TH, B * parts); }
+// (the parts beside the tiles: the batch alone may fill the grid's z, 65,535)
+dim3 conv_grid(int H, int W, int B, int parts = 1) { return dim3((W + TW - 1) / TW * parts, (H + TH - 1) / TH, B); }
 
 // ── fused inference on the tensor cores (tcgen05, BF16 operands, FP32 accumulation) ──
 // One CTA computes a 32x16 tile of outputs.  The three layers run over the
@@ -901,7 +902,7 @@ static int train_alloc(TrainBuf& t, int nb, int P) {
 // the batch already in t (u, m, ewt, x, mask, gam)
 static int train_fwd_bwd(cudaStream_t s, const float* w, float* g, TrainBuf& t, int nb, int P, double* loss) {
   const dim3 cg = conv_grid(P, P, nb, 3), cd = conv_grid(P, P, nb, conv_parts(CH)), cb(TW, TH);
-  const int nblk = cg.x * cg.y * nb;
+  const int nblk = cg.x / 3 * cg.y * nb;
   const size_t pl = (size_t)nb * P * P;
   const int eg = (int)std::min<size_t>((pl + 255) / 256, 4096);
   LLG_COUNT(KID_LEARNED);
