@@ -629,7 +629,10 @@ int demag64_create(llg_ctx* c, int px, int py, int hx, int ng, int ny, int open,
   klaunch(k_tensor_half, c->num_sms * 8, 256, 0, c->stream, txx, tyy, tzz, txy, py, hx, d->th);
   if (!open) cudaMemcpyAsync(d->txy, txy, sizeof(dcx) * nf, cudaMemcpyDeviceToDevice, c->stream);
   pdl_break();
-  if (cudaPeekAtLastError() != cudaSuccess) return fail(LLG_ERR_CUDA);
+  if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) {
+    llg_set_error(std::string("demag: tensor spectra: ") + cudaGetErrorString(e));
+    return fail(LLG_ERR_CUDA);
+  }
   const int rc = demag64_tune(c, d, c->d_hd, c->d_pm);
   if (rc) return fail(rc);
   *out = d;

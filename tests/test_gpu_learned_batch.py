@@ -29,3 +29,18 @@ def test_large_batch(gpu):
     assert abs(loss - loss0) <= 1e-12 * abs(loss0)
     assert np.array_equal(z.reshape(reps, *z0.shape), np.broadcast_to(z0, (reps,) + z0.shape))
     assert np.abs(grad - grad0).max() <= 2.0 ** -23 * np.abs(grad0).max()
+
+
+def test_a_refused_launch_fails_its_own_call_only(gpu):
+    """65,536 patches exceed the grid's z limit: the call reports the refused
+    launch, and the next one, on a context of its own, does not see it."""
+    import torch
+    ctx = llg.Context(llg.default_params(32, 16))
+    y = torch.ones(3 * 32 * 16, dtype=torch.float64, device=gpu)
+    f = torch.zeros_like(y)
+    w = np.zeros(llg.LEARNED_NWEIGHTS, np.float32)
+    b = {k: np.repeat(v, 65536, axis=0) for k, v in _patches(1, 8).items()}
+    with pytest.raises(llg.LLGError):
+        llg.learned_loss_grad(w, b["u"], b["m"], b["mask"], b["ewt"], b["x"], b["gamma"])
+    ctx.rhs(0.0, y, f)
+    torch.cuda.synchronize()
