@@ -1241,6 +1241,12 @@ struct Integrator {
   }
 };
 
+void integrator_destroy(Integrator* b) {
+  if (!b) return;
+  b->free_all();
+  delete b;
+}
+
 int integrator_create(llg_ctx* c, double t0, const double* y0, const llg_solver_opts* o) {
   Integrator* b = new Integrator();
   b->c = c;
@@ -1269,8 +1275,9 @@ int integrator_create(llg_ctx* c, double t0, const double* y0, const llg_solver_
   // The vectors of the integrator that this one replaces are taken over where
   // both have them (the context's grid, so their length, does not change): a
   // film of 1536x512 holds 17 vectors of 18.9 MB, whose cudaMalloc and cudaFree
-  // cost 8 to 200 ms per call here against some 60 us for clearing them.  Until
-  // everything that can fail has succeeded, the old integrator is untouched.
+  // cost 8 to 200 ms per call here against some 60 us for clearing them.  A call
+  // that fails up to the copy of y0 leaves the old integrator as it was; the
+  // clearing overwrites its vectors, so if that fails the context has none.
   Integrator* const old = c->integ;
   std::vector<std::pair<double**, double**>> vs;   // (this one's, the old one's)
   for (int j = 0; j <= b->qmax; j++) vs.push_back({&b->zn[j], old ? &old->zn[j] : nullptr});
@@ -1295,17 +1302,25 @@ int integrator_create(llg_ctx* c, double t0, const double* y0, const llg_solver_
   // work of the old integrator on another stream may still use its vectors
   if (old && old->stream != c->stream && cudaDeviceSynchronize() != cudaSuccess) {
     llg_set_error("integrator_init: device synchronisation failed");
+    cudaGetLastError();
     return fail(LLG_ERR_CUDA);
   }
   double* const z0 = b->zn[0] ? b->zn[0] : old->zn[0];
   if (y0 && cudaMemcpyAsync(z0, y0, vb, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess) {
     llg_set_error("integrator_init: copy of y0 failed");
+    cudaGetLastError();
     return fail(LLG_ERR_CUDA);
   }
-  for (auto& v : vs) {
+  for (auto& v : vs)
     if (!*v.first) std::swap(*v.first, *v.second);
-    if (!(y0 && v.first == &b->zn[0])) LLG_CUDA_TRY(cudaMemsetAsync(*v.first, 0, vb, c->stream));
-  }
+  integrator_destroy(old);
+  c->integ = nullptr;
+  for (auto& v : vs)
+    if (!(y0 && v.first == &b->zn[0]) && cudaMemsetAsync(*v.first, 0, vb, c->stream) != cudaSuccess) {
+      llg_set_error("integrator_init: clearing of the vectors failed");
+      cudaGetLastError();
+      return fail(LLG_ERR_CUDA);
+    }
   b->stream = c->stream;
   b->tn = t0;
   b->q = 1;
@@ -1313,7 +1328,6 @@ int integrator_create(llg_ctx* c, double t0, const double* y0, const llg_solver_
   b->qwait = b->L;
   b->etamax = ETAMX1;
   b->indx_acor = b->qmax;
-  if (c->integ) { c->integ->free_all(); delete c->integ; }
   c->integ = b;
   c->red_per = (b->kf32_req || c->p.demag_precision == LLG_DEMAG_MIXED) ? 8 : 1;   // see red_blocks
   // the FP32-basis operator reads an FP32 block inverse: psetup stores that
@@ -1323,12 +1337,6 @@ int integrator_create(llg_ctx* c, double t0, const double* y0, const llg_solver_
     c->have_setup = 0;
   }
   return 0;
-}
-
-void integrator_destroy(Integrator* b) {
-  if (!b) return;
-  b->free_all();
-  delete b;
 }
 
 int integrator_run(llg_ctx* c, double tout, double* yout, double* tret) {
