@@ -428,9 +428,10 @@ __global__ void __launch_bounds__(FNT, 2) k_learned_fused(InferArgs a) {
   double acc[1] = {0.0};
   bool good = true;
   // Tiles without an active cell in their input region (listed after the live
-  // ones): their features, and so the network's output, are exactly zero
-  // (linear, no bias), so the three layers are left out and the output keeps
-  // the expression of the general path; one cell per thread, no barrier.
+  // ones): their features, and so the output of a network of finite weights,
+  // are exactly zero (linear, no bias), so the three layers are left out and
+  // the output keeps the expression of the general path; one cell per thread, no
+  // barrier.
   static_assert(FO_W * FO_H == FNT, "one output cell per thread");
   const int nlive = a.tiles ? a.tiles[0] : a.ntiles;
   for (int it = nlive + blockIdx.x; it < a.ntiles; it += gridDim.x) {
@@ -636,6 +637,7 @@ struct Learned {
   float* d_m1 = nullptr;
   float* d_m2 = nullptr;
   bool have_weights = false;
+  bool finite = false;       // every weight is, as BF16 too
   int fell_back = 0;         // block-Jacobi fallback: 1 failed solve, 2 not worth its cost
   double pol_it_learned = -1.0, pol_it_bj = -1.0, pol_kappa = -1.0;   // last policy judgement
   int policy = 1;            // 1: cost-aware probing, 0: learned on every solve
@@ -777,8 +779,10 @@ int learned_apply(llg_ctx* c, const double* ewt, double* out, int slot, const do
     a.ng = c->p.ng; a.ny = c->p.ny;
     a.ntx = (c->p.ng + FO_W - 1) / FO_W;
     a.ntiles = a.ntx * ((c->p.ny + FO_H - 1) / FO_H);
-    if ((rc = ensure_tiles(c, l, a.ntx, a.ntiles))) return rc;
-    a.tiles = c->d_act ? l->d_tiles : nullptr;
+    if (l->finite) {   // (a NaN weight shows in every cell)
+      if ((rc = ensure_tiles(c, l, a.ntx, a.ntiles))) return rc;
+      a.tiles = c->d_act ? l->d_tiles : nullptr;
+    }
     a.partials = c->d_red; a.counter = c->d_counter;
     a.res = slot >= 0 ? c->d_scal + slot : nullptr;
     a.err = l->d_err;
@@ -957,6 +961,13 @@ int llg_learned_harvest(llg_ctx* c, int32_t max_samples, int32_t stride) {
   return 0;
 }
 
+// whether all weights are finite, rounded to BF16 (maximum 3.39e38) too
+static bool weights_finite(const float* w) {
+  for (int i = 0; i < NWT; i++)
+    if (!(fabsf(w[i]) < 3.38e38f)) return false;
+  return true;
+}
+
 int llg_learned_num_samples(llg_ctx* c) { return (c && c->learned) ? c->learned->nsamples : 0; }
 
 int llg_learned_set_weights(llg_ctx* c, const float* h_w, int32_t n) {
@@ -969,6 +980,7 @@ int llg_learned_set_weights(llg_ctx* c, const float* h_w, int32_t n) {
   k_pack_weights<<<(27 * 256 + 255) / 256, 256, 0, c->stream>>>(l->d_w, l->d_wpack);
   LLG_CUDA_TRY(cudaPeekAtLastError());
   LLG_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  l->finite = weights_finite(h_w);
   l->have_weights = true;
   l->fell_back = 0;
   return 0;
@@ -1110,8 +1122,11 @@ int llg_learned_train(llg_ctx* c, const llg_train_opts* o, double* loss_first, d
   }
   k_round_bf16<<<(NWT + 255) / 256, 256, 0, s>>>(l->d_w, l->d_wq, NWT);
   k_pack_weights<<<(27 * 256 + 255) / 256, 256, 0, s>>>(l->d_w, l->d_wpack);
+  std::vector<float> hw(NWT);
+  LLG_CUDA_TRY(cudaMemcpyAsync(hw.data(), l->d_w, sizeof(float) * NWT, cudaMemcpyDeviceToHost, s));
   LLG_CUDA_TRY(cudaStreamSynchronize(s));
   t.release();
+  l->finite = weights_finite(hw.data());
   l->have_weights = true;
   l->fell_back = 0;
   return 0;
