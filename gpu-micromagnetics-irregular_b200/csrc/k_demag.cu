@@ -822,10 +822,19 @@ void demag_destroy(DemagPlan* d) {
   delete d;
 }
 
+// The limit belongs to the kernel, not to the plan: only ever raised, since
+// plans of longer transforms may be alive.
 static int set_smem(const void* fn, size_t bytes) {
-  if (bytes > 48 * 1024) {
-    LLG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  }
+  if (bytes <= 48 * 1024) return 0;
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> limit;   // (device, kernel)
+  int dev = 0;
+  LLG_CUDA_TRY(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> g(mu);
+  size_t& cur = limit[{dev, fn}];
+  if (bytes <= cur) return 0;
+  LLG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  cur = bytes;
   return 0;
 }
 

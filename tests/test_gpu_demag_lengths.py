@@ -29,3 +29,27 @@ def test_field_matches_the_oracle(gpu, oracle_lib, ng, ny, opened, precision):
     llg.Context(p).demag_apply(torch.from_numpy(y).to(gpu), h)
     # the bounds of the two chains' other field tests
     assert rel_err(h.cpu().numpy(), want) <= (1e-11 if precision == llg.DEMAG_FP64 else 5e-6)
+
+
+@pytest.mark.parametrize("shape", [lambda n: (8, n), lambda n: (n, 8)], ids=["columns", "rows"])
+def test_a_longer_plan_outlives_a_shorter_one(gpu, shape):
+    """A kernel's shared-memory limit is process-wide: the plan of a shorter
+    transform must not lower it under a longer one's."""
+    import torch
+
+    def context(n):
+        ng, ny = shape(n)
+        ctx = llg.Context(llg.default_params(ng, ny, demag_mode=llg.DEMAG_PERIODIC, demag_strength=1.0,
+                                             demag_precision=llg.DEMAG_MIXED))
+        y = torch.from_numpy(np.random.default_rng(n).uniform(-1.0, 1.0, 3 * ng * ny)).to(gpu)
+        return ctx, y, torch.zeros_like(y)
+
+    lengths = (4000, 3000) if shape(1) == (8, 1) else (8100, 6400)   # all above 48 KB a block
+    a = context(lengths[0])
+    a[0].demag_apply(a[1], a[2])
+    want = a[2].clone()
+    b = context(lengths[1])
+    b[0].demag_apply(b[1], b[2])
+    a[2].zero_()
+    a[0].demag_apply(a[1], a[2])
+    assert torch.equal(a[2], want)
