@@ -37,7 +37,7 @@ struct IpPlan {
   const double2* tw;
 };
 
-// radices with an in-register DFT here (a prime from 17 to 61: ip_pass_warp)
+// radices with an in-register DFT here (a prime from 17 to 61: ip_mid_group)
 __host__ __device__ constexpr bool ip_radix(int r) {
   return r == 1 || r == 2 || r == 3 || r == 4 || r == 5 || r == 6 || r == 7 || r == 8 || r == 9 || r == 10 ||
          r == 11 || r == 12 || r == 13 || r == 15 || r == 16;
@@ -354,52 +354,66 @@ FFT_HD void ip_mid(dcx* buf, int bs, int nb, const dcx* tw, int n, int r0, int S
     for (int r = 0; r < RAD; r++) p[r * Lr] = v[r];
   }
 }
-// a middle pass of prime radix 17..61: one warp per butterfly, lane l forms
-// the outputs l and l + 32 from the butterfly's values in shared memory
-// (broadcast reads); only the warp's own values are touched, so __syncwarp
-// separates reads from writes
-template <int SIGN>
-__device__ __noinline__ void ip_mid_warp(dcx* buf, int bs, int nb, const dcx* __restrict__ tw, int n, int r0, int S,
-                                         int L, int RAD, int tid, int T) {
-  const int Lr = L / RAD, per = n / RAD, ts = n / L, rs = n / RAD;
-  const int lane = tid & 31;
-  for (int q = tid >> 5; q < per * nb; q += T >> 5) {
+// A middle pass of prime radix R, 17..61: a butterfly per group of GL lanes (16
+// up to 31, else 32), which fold the values into sums and differences of v[r] and
+// v[R-r] in place; lane l then forms the outputs l and R-l from the (R-1)/2 pairs
+// (broadcast reads), a quarter of the products of the plain sums.  Only the
+// group's own values are touched, so __syncwarp separates reads from writes.
+// Against a warp per butterfly and plain sums, which on filled grids ran behind the
+// autosort pass of a thread per butterfly: field of 348x512 open (a factor 29) 138
+// us autosort, 193 plain, 70 now; 256x361 (19, 19) 135, 172, 64; 1450x1024 915, 1045, 472.
+template <int SIGN, int GL>
+__device__ __noinline__ void ip_mid_group(dcx* buf, int bs, int nb, const dcx* __restrict__ tw, int n, int r0, int S,
+                                          int L, int RAD, int tid, int T) {
+  constexpr int G = 32 / GL;   // groups of a warp
+  const int Lr = L / RAD, per = n / RAD, ts = n / L, rs = n / RAD, H = (RAD - 1) / 2;
+  const int l = tid % GL, total = per * nb;
+  for (int q0 = (tid >> 5) * G; q0 < total; q0 += (T >> 5) * G) {   // (the same for all lanes of a warp)
+    const int q = q0 + (tid & 31) / GL;
+    const bool in = q < total && l <= H;
     const int b = q / per, x = q - b * per;
     const int y = x / r0, d0 = x - y * r0;
     const int blk = y / Lr, j = y - blk * Lr;
     dcx* p = buf + b * bs + d0 * S + blk * L + j;
-    if constexpr (SIGN > 0) {   // twiddles first, in place
-      for (int r = lane; r < RAD; r += 32) {
-        dcx w = __ldg(&tw[r * j * ts]);
-        w.y = -w.y;
-        p[r * Lr] = cmul<double>(p[r * Lr], w);
+    auto twiddled = [&](dcx v, int r) {
+      dcx w = __ldg(&tw[r * j * ts]);
+      if (SIGN > 0) w.y = -w.y;
+      return cmul<double>(v, w);
+    };
+    dcx s = mk<double>(0.0, 0.0), t = s;
+    if (in) s = p[0];
+    if (in && l > 0) {
+      dcx u = p[l * Lr], v = p[(RAD - l) * Lr];
+      if constexpr (SIGN > 0) {   // twiddles first
+        u = twiddled(u, l);
+        v = twiddled(v, RAD - l);
       }
-      __syncwarp();
+      p[l * Lr] = cadd<double>(u, v);
+      p[(RAD - l) * Lr] = csub<double>(u, v);
     }
-    dcx o[2];
-    int e[2] = {0, 0};
-    const int k[2] = {lane < RAD ? lane : 0, lane + 32 < RAD ? lane + 32 : 0};
-    o[0] = o[1] = mk<double>(0.0, 0.0);
-    for (int r = 0; r < RAD; r++) {
-      const dcx v = p[r * Lr];
-#pragma unroll
-      for (int u = 0; u < 2; u++) {
-        dcx w = __ldg(&tw[e[u] * rs]);
-        if (SIGN > 0) w.y = -w.y;
-        o[u].x += v.x * w.x - v.y * w.y;
-        o[u].y += v.x * w.y + v.y * w.x;
-        e[u] += k[u];
-        if (e[u] >= RAD) e[u] -= RAD;
+    __syncwarp();
+    if (in) {
+      int e = 0;
+#pragma unroll 4
+      for (int r = 1; r <= H; r++) {
+        e += l;
+        if (e >= RAD) e -= RAD;   // (r l) mod R
+        const dcx u = p[r * Lr], d = p[(RAD - r) * Lr], w = __ldg(&tw[e * rs]);   // cos, -sin
+        s.x += w.x * u.x;
+        s.y += w.x * u.y;
+        t.x += w.y * d.x;
+        t.y += w.y * d.y;
       }
     }
     __syncwarp();
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const int kk = lane + 32 * u;
-      if (kk < RAD) {
-        if constexpr (SIGN < 0) o[u] = cmul<double>(o[u], __ldg(&tw[kk * j * ts]));
-        p[kk * Lr] = o[u];
+    if (in) {
+      dcx o = mk<double>(s.x + SIGN * t.y, s.y - SIGN * t.x), m = mk<double>(s.x - SIGN * t.y, s.y + SIGN * t.x);
+      if constexpr (SIGN < 0) {
+        o = twiddled(o, l);
+        m = twiddled(m, RAD - l);
       }
+      p[l * Lr] = o;
+      if (l > 0) p[(RAD - l) * Lr] = m;
     }
     __syncwarp();
   }
@@ -438,7 +452,7 @@ double pass_cost(int r) {
     case 13: return 30;
     case 15: return 18;
     case 16: return 16.5;
-    default: return 6.0 * r;   // one warp per butterfly
+    default: return 6.0 * r;   // ip_mid_group
   }
 }
 constexpr double kSweep = 10;   // a pass's shared-memory sweep and barrier, in the same unit

@@ -173,7 +173,9 @@ struct DynPlan {
     break;
       LLG_IP_CASES(K)
 #undef K
-      default: ip_mid_warp<SIGN>(buf, s, nb, p.tw, p.n, p.r[0], p.S, L, R, tid, T);
+      default:
+        if (R < 32) ip_mid_group<SIGN, 16>(buf, s, nb, p.tw, p.n, p.r[0], p.S, L, R, tid, T);
+        else ip_mid_group<SIGN, 32>(buf, s, nb, p.tw, p.n, p.r[0], p.S, L, R, tid, T);
     }
   }
   __device__ __forceinline__ void mids_fwd(dcx* buf, int nb, int tid, int T) const {

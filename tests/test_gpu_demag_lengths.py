@@ -53,3 +53,17 @@ def test_a_longer_plan_outlives_a_shorter_one(gpu, shape):
     a[2].zero_()
     a[0].demag_apply(a[1], a[2])
     assert torch.equal(a[2], want)
+
+
+@pytest.mark.parametrize("ng,ny", [(17, 29), (19, 23), (31, 37), (41, 43), (47, 59), (3 * 29, 2 * 31), (1, 37), (870, 37),
+                                   (61, 1054)])
+def test_prime_passes_of_the_fp64_chain(gpu, oracle_lib, ng, ny):
+    """A group of 16 lanes per butterfly up to 31, of 32 from 37 on: odd numbers of
+    butterflies, fewer than a warp's groups, and many per thread block."""
+    import torch
+    p = llg.default_params(ng, ny, demag_mode=llg.DEMAG_PERIODIC, demag_strength=2.5)
+    y = np.random.default_rng(ng + ny).uniform(-1.0, 1.0, 3 * ng * ny)
+    want = oracle_lib.Oracle(p).demag(y)
+    h = torch.full((3 * ng * ny,), float("nan"), dtype=torch.float64, device=gpu)
+    llg.Context(p).demag_apply(torch.from_numpy(y).to(gpu), h)
+    assert rel_err(h.cpu().numpy(), want) <= 1e-11
