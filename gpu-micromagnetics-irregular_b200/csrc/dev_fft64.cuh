@@ -420,19 +420,25 @@ __device__ __noinline__ void ip_mid_group(dcx* buf, int bs, int nb, const dcx* _
 }
 
 // ── plans (host) ──
-// Lengths whose kernels are instantiated with constant radices (the
-// benchmark films' and the powers of two between 128 and 4096).  Every other
-// length reads its radices from the plan: the same passes, with integer
-// divisions for the slots and a branch per pass.
+// Lengths whose kernels are instantiated with constant radices: the 2^k from 32
+// to 4096 and the 3 2^k from 48 to 3072, the powers of two that grids are made of
+// and one and a half times them.  Every other length reads its radices from the
+// plan: the same passes, with integer divisions for the slots and a branch per
+// pass, at about half the speed (field, plan read / constant: 32x32 periodic 16.5 /
+// 8.3 us, 512x512 31 / 16.5, 2048x2048 330 / 172, 1536x512 open 148 / 76).
 //   rows: the radix fused with the packing is the large one (its two groups
-//   stay in registers, which saves a sweep); columns: the fused one is 4, since
-//   three components' butterflies share the registers there.
-#define LLG_ROWS64(M) \
-  M(128, 8, 4, 1, 4) M(256, 8, 8, 1, 4) M(512, 16, 8, 1, 4) M(1024, 16, 16, 1, 4) M(1536, 16, 16, 1, 6) \
-  M(2048, 16, 16, 1, 8) M(3072, 16, 16, 1, 12) M(4096, 16, 16, 4, 4)
-#define LLG_COLS64(M) \
-  M(128, 8, 4, 1, 4) M(256, 16, 4, 1, 4) M(512, 16, 8, 1, 4) M(1024, 16, 16, 1, 4) M(2048, 16, 8, 4, 4) \
-  M(4096, 16, 16, 4, 4)
+//   stay in registers, which saves a sweep); columns: the fused one is 6 at
+//   most, since three components' butterflies share the registers there.
+#define LLG_ROWS64(M)                                                                            \
+  M(32, 8, 1, 1, 4) M(64, 16, 1, 1, 4) M(128, 8, 4, 1, 4) M(256, 8, 8, 1, 4) M(512, 16, 8, 1, 4) \
+  M(1024, 16, 16, 1, 4) M(2048, 16, 16, 1, 8) M(4096, 16, 16, 4, 4)                              \
+  M(48, 8, 1, 1, 6) M(96, 16, 1, 1, 6) M(192, 16, 1, 1, 12) M(384, 16, 4, 1, 6)                  \
+  M(768, 16, 8, 1, 6) M(1536, 16, 16, 1, 6) M(3072, 16, 16, 1, 12)
+#define LLG_COLS64(M)                                                                             \
+  M(32, 8, 1, 1, 4) M(64, 16, 1, 1, 4) M(128, 8, 4, 1, 4) M(256, 16, 4, 1, 4) M(512, 16, 8, 1, 4) \
+  M(1024, 16, 16, 1, 4) M(2048, 16, 8, 4, 4) M(4096, 16, 16, 4, 4)                                \
+  M(48, 16, 1, 1, 3) M(96, 16, 1, 1, 6) M(192, 16, 4, 1, 3) M(384, 16, 6, 1, 4)                   \
+  M(768, 16, 12, 1, 4) M(1536, 16, 16, 1, 6) M(3072, 16, 16, 3, 4)
 
 // instruction weight per element of one pass of radix r, twiddles included
 double pass_cost(int r) {

@@ -55,6 +55,24 @@ def test_a_longer_plan_outlives_a_shorter_one(gpu, shape):
     assert torch.equal(a[2], want)
 
 
+@pytest.mark.parametrize("n", [32, 48, 64, 96, 192, 384, 768, 1536, 3072])
+@pytest.mark.parametrize("opened", [0, 1])
+@pytest.mark.parametrize("columns", [0, 1])
+def test_constant_plans_of_the_fp64_chain(gpu, oracle_lib, n, opened, columns):
+    """Lengths with constant radices that the other tests leave out, in rows and in
+    columns: two passes, a fused radix of 12, three middle passes."""
+    ng, ny = (n // 2 if opened else n), 5
+    if columns:
+        ng, ny = ny, ng
+    import torch
+    p = llg.default_params(ng, ny, demag_mode=llg.DEMAG_OPEN if opened else llg.DEMAG_PERIODIC, demag_strength=2.5)
+    y = np.random.default_rng(ng + ny).uniform(-1.0, 1.0, 3 * ng * ny)
+    want = oracle_lib.Oracle(p).demag(y)
+    h = torch.full((3 * ng * ny,), float("nan"), dtype=torch.float64, device=gpu)
+    llg.Context(p).demag_apply(torch.from_numpy(y).to(gpu), h)
+    assert rel_err(h.cpu().numpy(), want) <= 1e-11
+
+
 @pytest.mark.parametrize("ng,ny", [(17, 29), (19, 23), (31, 37), (41, 43), (47, 59), (3 * 29, 2 * 31), (1, 37), (870, 37),
                                    (61, 1054)])
 def test_prime_passes_of_the_fp64_chain(gpu, oracle_lib, ng, ny):
