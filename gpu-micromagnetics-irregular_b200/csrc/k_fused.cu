@@ -418,9 +418,11 @@ __global__ void __launch_bounds__(RT) k_wrms2(const double* __restrict__ x1, dou
 // zn[j] *= f_j, j = 1..Q; the Nordsieck predictor (Pascal triangle); and y =
 // normalise(zn0 + 0), the first Newton iterate's state.  Per element the
 // arithmetic of k_ewt_wrms, k_scale_cols, k_nordsieck and k_lin_normalize.
-// Every load of a cell is issued before its first store.
+// Every load of a cell is issued before its first store.  Blocks per SM as in
+// gs_resident: the weights' sums are added over them.
+constexpr int predict_resident(int q) { return q <= 2 ? 4 : q <= 4 ? 3 : 2; }
 template <int Q>
-__global__ void __launch_bounds__(RT) k_predict_fused(ZPack zn, CPack f, int pend, int do_ewt, double rtol,
+__global__ void __launch_bounds__(RT, predict_resident(Q)) k_predict_fused(ZPack zn, CPack f, int pend, int do_ewt, double rtol,
                                                       double atol, double* __restrict__ ewt, double* __restrict__ y,
                                                       int n, int kind, double eps, double* partials,
                                                       unsigned int* counter, double* out, int lazy, CPack lc,
@@ -745,7 +747,7 @@ int fused_predict(llg_ctx* c, int q, double* const* zn, const double* f, bool pe
   const int pe = pend ? 1 : 0, de = do_ewt ? 1 : 0;
   double* out = c->d_scal + slot;
 #define PRED(Q)                                                                                                \
-  klaunch(k_predict_fused<Q>, cap_resident(nb, LLG_PER_SM((k_predict_fused<Q>)), c->num_sms), RT, 0, c->stream,  \
+  klaunch(k_predict_fused<Q>, cap_resident(nb, predict_resident(Q), c->num_sms), RT, 0, c->stream,  \
           zp, fp, pe, de, rtol, atol, ewt, y, c->ncell, c->p.norm_kind,                                          \
                                                c->p.norm_eps, c->d_red, c->d_counter, out, lz, lp, acor,         \
                                                lz ? zsave : nullptr)

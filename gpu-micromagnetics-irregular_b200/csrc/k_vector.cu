@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(RT) k_gs_update(int k, VPack<VT> X, const doub
   __syncthreads();
   double cf[MAXV - 1];
 #pragma unroll
-  for (int j = 0; j < MAXV - 1; j++) cf[j] = (j < k) ? -slot_value(dots + j) : 0.0;
+  for (int j = 0; j < MAXV - 1; j++) cf[j] = (j < k) ? -dots[j] : 0.0;
   double acc[1] = {0.0};
   const long long st = (long long)gridDim.x * RT;
   for (long long i0 = blockIdx.x * (long long)RT + threadIdx.x; i0 < n; i0 += UB * st) {
@@ -307,10 +307,17 @@ __global__ void __launch_bounds__(RT) k_gs_update(int k, VPack<VT> X, const doub
 // all K basis vectors (and of z) for the UB slice elements are issued before
 // any of them is used, where the runtime-k loop waits on one vector at a
 // time.  Per element the same operations in the same order, so z is bitwise
-// that of k_gs_update; it runs on one resident wave of blocks
-// (red_blocks_resident), so its sum of squares is added in another partition.
+// that of k_gs_update; it runs on one resident wave of blocks (gs_resident per
+// SM), so its sum of squares is added in another partition.  The partition is
+// part of the result: the launch bounds hold the kernel to the count, whatever
+// registers the compiler would take.
 template <int K, typename VT>
-__global__ void __launch_bounds__(RT) k_gs_update_k(VPack<VT> X, const double* dots, VT* z, long long n,
+constexpr int gs_resident() {
+  constexpr int fp64[8] = {6, 6, 5, 5, 4, 4, 4, 3}, fp32[8] = {8, 6, 5, 4, 4, 4, 3, 3};
+  return (sizeof(VT) == 8 ? fp64 : fp32)[K - 1];
+}
+template <int K, typename VT>
+__global__ void __launch_bounds__(RT, gs_resident<K, VT>()) k_gs_update_k(VPack<VT> X, const double* dots, VT* z, long long n,
                                                     double* partials, unsigned int* counter, double* out, KScale ks,
                                                     double* aout, Pub pub) {
   pdl_entry();
@@ -321,7 +328,7 @@ __global__ void __launch_bounds__(RT) k_gs_update_k(VPack<VT> X, const double* d
   double cf[K], xa[K];
 #pragma unroll
   for (int j = 0; j < K; j++) {
-    cf[j] = -slot_value(dots + j);
+    cf[j] = -dots[j];
     xa[j] = xs[j];
   }
   double acc[1] = {0.0};
@@ -368,7 +375,7 @@ __global__ void __launch_bounds__(RT) k_mgs_step(const double* __restrict__ X, c
                                                  Pub pub) {
   pdl_entry();
   __shared__ double sm[RT / 32];
-  const double h = slot_value(hd), xa = kscale_of(xa_p), ya = kscale_of(ya_p);
+  const double h = *hd, xa = kscale_of(xa_p), ya = kscale_of(ya_p);
   double acc[1] = {0.0};
   const long long st = (long long)gridDim.x * RT;
   for (long long i0 = blockIdx.x * (long long)RT + threadIdx.x; i0 < n; i0 += UB * st) {
@@ -392,7 +399,7 @@ __global__ void __launch_bounds__(RT) k_mgs_step(const double* __restrict__ X, c
   }
   block_sum<1>(acc, sm);
   const bool last = finalize<1>(partials, gridDim.x, counter, out, 0, 1.0, acc);
-  if (last && aout && threadIdx.x == 0) *aout = mgs_scale_of(out[0], slot_value(vk));
+  if (last && aout && threadIdx.x == 0) *aout = mgs_scale_of(out[0], *vk);
   if (last) publish_carried(pub);
 }
 
@@ -563,7 +570,7 @@ static int vgs_update_impl(llg_ctx* c, int k, VT* const* V, int slot_dots, int s
   const KScale kk = ks ? *ks : kz;
   const Pub pub = take_publish(c);
 #define GS_K(K)                                                                                                  \
-  klaunch(k_gs_update_k<K, VT>, red_blocks_resident(c->neq, c->red_per, LLG_PER_SM((k_gs_update_k<K, VT>)), c->num_sms), RT, \
+  klaunch(k_gs_update_k<K, VT>, red_blocks_resident(c->neq, c->red_per, gs_resident<K, VT>(), c->num_sms), RT, \
           0, c->stream, pk, dots, V[k], c->neq, c->d_red, c->d_counter, ss, kk, aout, pub)
   switch (k) {
     case 1: GS_K(1); break;

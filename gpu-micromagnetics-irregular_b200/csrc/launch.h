@@ -21,11 +21,11 @@
 // place, and its blocks' shares meet inside a 32-byte sector (components of an
 // odd number of cells, spectrum columns of an odd height, scalar slots next to
 // one another).  griddepcontrol.wait covers ordinary loads, not the non-coherent
-// path, so such data is read past L1 (__ldcg) on one side at least: by the
+// path, so such vectors are read past L1 (__ldcg) on one side at least: by the
 // in-place kernels whose shares can meet so (k_normalize, k_predict_fused), by
-// the readers of the spectrum (k_rows_inv, k_rows_inv64), and in every load of a
-// scalar slot (slot_value).  The other in-place kernels' blocks own whole
-// 256-element slices of vectors that start on 256 bytes.
+// the readers of the spectrum (k_rows_inv, k_rows_inv64); scalar slots are read
+// with ordinary loads.  The other in-place kernels' blocks own whole 256-element
+// slices of vectors that start on 256 bytes.
 //
 // A PDL launch relaxes the dependency on the preceding kernel only, so it is
 // used only where every operation of the stream between two such kernels is

@@ -247,14 +247,13 @@ struct KScale {
   const double* a[KS_MAX];
 };
 #ifdef __CUDACC__
-// a device scalar, past L1 (launch.h: the kernel before may have read another
-// slot of its line)
-__device__ __forceinline__ double slot_value(const double* a) { return __ldcg(a); }
-__device__ __forceinline__ double kscale_of(const double* a) { return a ? slot_value(a) : 1.0; }
+// (scalar slots are read with ordinary loads, never through a const __restrict__
+// pointer: launch.h)
+__device__ __forceinline__ double kscale_of(const double* a) { return a ? *a : 1.0; }
 // scale of a vector with sum of squares ss; vk (optional): its sum of squares
 // before the Gram-Schmidt update (1000 ||v|| < ||v before||: a second pass is due)
 __device__ __forceinline__ double gs_scale_of(double ss, const double* vk) {
-  if (vk && 1000.0 * sqrt(ss) < sqrt(slot_value(vk))) return 1.0;
+  if (vk && 1000.0 * sqrt(ss) < sqrt(*vk)) return 1.0;
   return 1.0 / sqrt(ss);
 }
 // the same after modified Gram-Schmidt, whose second pass is due when ||v||
