@@ -440,7 +440,9 @@ __device__ __noinline__ void ip_mid_group(dcx* buf, int bs, int nb, const dcx* _
   M(48, 16, 1, 1, 3) M(96, 16, 1, 1, 6) M(192, 16, 4, 1, 3) M(384, 16, 6, 1, 4)                   \
   M(768, 16, 12, 1, 4) M(1536, 16, 16, 1, 6) M(3072, 16, 16, 3, 4)
 
-// instruction weight per element of one pass of radix r, twiddles included
+// instruction weight per element of one pass of radix r, twiddles included:
+// counted from the code above and only used to rank factorisations of the same
+// length (a prime's weight never decides, its pass is given)
 double pass_cost(int r) {
   switch (r) {
     case 1: return 0;
@@ -461,7 +463,7 @@ double pass_cost(int r) {
     default: return 6.0 * r;   // ip_mid_group
   }
 }
-constexpr double kSweep = 10;   // a pass's shared-memory sweep and barrier, in the same unit
+constexpr double kSweep = 10;   // a pass's shared-memory sweep and barrier, in the same unit (an estimate)
 
 // cheapest middle passes for what is left of the length
 void search_mids(int left, int from, std::vector<int>& cur, double cost, double& best, std::vector<int>& out) {

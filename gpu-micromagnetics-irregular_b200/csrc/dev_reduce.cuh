@@ -28,7 +28,7 @@ constexpr int RMAXB = 1024;     // max reduction blocks
 // llg.h, whose sums callers may compare between contexts, and integrators with
 // FP32 parts, whose trajectories turn another rounding of a sum into other
 // FP32 values.
-constexpr int RED_PER = 8;
+// (RED_PER, llg_internal.h.)
 int red_blocks(long long n, int per) {
   long long b = (n + RT * per - 1) / (RT * per);
   if (b > RMAXB) b = RMAXB;

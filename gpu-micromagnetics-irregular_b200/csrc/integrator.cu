@@ -1329,7 +1329,7 @@ int integrator_create(llg_ctx* c, double t0, const double* y0, const llg_solver_
   b->etamax = ETAMX1;
   b->indx_acor = b->qmax;
   c->integ = b;
-  c->red_per = (b->kf32_req || c->p.demag_precision == LLG_DEMAG_MIXED) ? 8 : 1;   // see red_blocks
+  c->red_per = (b->kf32_req || c->p.demag_precision == LLG_DEMAG_MIXED) ? RED_PER : 1;   // see red_blocks
   // the FP32-basis operator reads an FP32 block inverse: psetup stores that
   // precision from now on (every step sequence starts with a setup)
   if (c->pinv_f32 != (b->kf32 ? 1 : 0)) {

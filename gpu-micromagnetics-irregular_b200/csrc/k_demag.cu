@@ -674,7 +674,7 @@ __global__ void k_tensor_finish(const double2* __restrict__ Sxx, const double2* 
 static constexpr int kRowsNB = 1;  // packed transforms per row-CTA at init (tensor spectra)
 
 // radices with an in-register DFT (stockham_pass); any other prime takes
-// the generic pass, one thread per butterfly
+// the generic pass, counted as one thread per butterfly
 static bool fixed_radix(int r) {
   return r == 2 || r == 3 || r == 4 || r == 5 || r == 6 || r == 8 || r == 12 || r == 16;
 }
@@ -768,7 +768,7 @@ static int fft_init(HostFft& f, int n, int batch) {
   for (int r : f.radix)
     if (!f.fix && !fixed_radix(r)) f.fix = -1;
   // threads per transform: n/16 covers the fixed radices (<= 16/R butterflies
-  // per thread); a generic radix R gets one thread per butterfly (n/R) at least.
+  // per thread); a generic radix R counts one thread per butterfly (n/R).
   f.ept = (((n + 7) / 8 + 31) / 32 * 32 * batch <= 1024) ? 8 : 16;
   int need = (n + f.ept - 1) / f.ept;
   for (int r : f.radix)

@@ -15,13 +15,13 @@
 // transform) and shared-memory sweeps, then the latency of each CTA's load;
 // HBM traffic is far below its roof.  The padded half of an open row or column
 // is neither loaded nor added, and its half of the last inverse pass is not
-// formed.  Measured at 1536x512 open (3072x1024 transforms), cold L2, against
-// the autosort kernels they replaced: rows_fwd 46.6 -> 24.5 us (16.8 of them
-// without the spectrum's stores), cols 96.3 -> 44 us, rows_inv 35.7 -> 30 us;
-// f of that film through the callbacks 205 -> 120 us, 375x225 open (750x450)
-// 43 -> 31 us for the field alone.  Radix 8 passes at twice the threads ran the
-// same times for rows and 53 us for columns; three and four resident CTAs
-// instead of two changed nothing, so the radix-16 forms stand.
+// formed.  1536x512 open (3072x1024 transforms), in the stream with the operands
+// in L2: rows_fwd 18.9 us, cols 36.6, rows_inv 18.5 (cold caches 27.7, 42.9, 38.4;
+// the autosort kernels before them 46.6, 96.3, 35.7 cold).  f of that film through
+// the callbacks 205 -> 107 us; 375x225 open (750x450), the field alone, 43 -> 28.6.
+// Radix 8 passes at twice the threads ran the same times for rows and 53 us for
+// columns; three and four resident CTAs instead of two changed nothing, so the
+// radix-16 forms stand.
 //
 // Tensor spectra: N_xx, N_yy, N_zz are even in the y frequency and, on the open
 // grid, N_xy is real and odd in it, so only ky = 0..n/2 is kept, interleaved

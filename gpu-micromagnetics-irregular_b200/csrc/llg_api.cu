@@ -98,7 +98,7 @@ static int validate(const llg_params* p) {
 struct PublicReduction {
   llg_ctx* c;
   int saved;
-  explicit PublicReduction(llg_ctx* ctx) : c(ctx), saved(ctx->red_per) { c->red_per = 8; }
+  explicit PublicReduction(llg_ctx* ctx) : c(ctx), saved(ctx->red_per) { c->red_per = RED_PER; }
   ~PublicReduction() { c->red_per = saved; }
 };
 

@@ -81,6 +81,8 @@ struct DevProblem {
   const double* nsk3;    // windowed
 };
 
+constexpr int RED_PER = 8;   // elements per thread of a reduction outside plain FP64 integrators (red_blocks)
+
 struct DemagPlan;   // k_demag.cu
 struct DemagTc;     // k_demag_tc.cu
 struct Demag64;     // k_demag64.cu
@@ -144,7 +146,7 @@ struct llg_ctx {
   Pub pub_armed{};              // requested, not yet given to a launch
   Pub pub_carried{};            // given to the last launch that took one
   int red_blocks_max = 0;
-  int red_per = 8;              // elements per thread of a reduction (red_blocks); set by integrator_create
+  int red_per = RED_PER;        // elements per thread of a reduction (red_blocks); set by integrator_create
 
   DemagPlan* demag = nullptr;
   Integrator* integ = nullptr;
